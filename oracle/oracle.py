@@ -17,7 +17,8 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 ORACLE_LIB = os.path.join(HERE, "liboracle.so")
 REF_LIB = os.path.join(HERE, "_ref", "libref_cpu.so")
 # Where the reference tree lies: $PATHED_REFERENCE, else the path the last build() was
-# given (recorded in _ref/REFERENCE_TREE), else None (tests that read it then skip).
+# given (recorded in _ref/REFERENCE_TREE), else a path that does not exist (tests that read
+# files there then skip).
 _TREE_NOTE = os.path.join(HERE, "_ref", "REFERENCE_TREE")
 
 
@@ -26,7 +27,7 @@ def _reference_tree():
     if not t and os.path.exists(_TREE_NOTE):
         with open(_TREE_NOTE) as f:
             t = f.read().strip()
-    return t or None
+    return t or os.path.join(HERE, "_ref", "no_reference_tree")
 
 
 REF_TREE = _reference_tree()
