@@ -63,32 +63,11 @@ __device__ __forceinline__ int warp_fetch(int* cursor, int n = 32) {
     return __shfl_sync(0xffffffffu, base, 0);
 }
 
-// Warp-aggregated append of up to N items per lane with one atomic per warp: slot[k] is the
-// slot of the lane's k-th item when want[k], -1 otherwise.
+// Warp-aggregated append to two queues whose lengths share one 64-bit counter (the low and the
+// high half; neither half ever exceeds a wave's 2^25 paths): one atomic per warp for both.
+// sa[k] / sb[k] are the lane's slots where wa[k] / wb[k], -1 otherwise.
 template <int N>
-__device__ __forceinline__ void warp_append_n(int* counter, const bool (&want)[N], int (&slot)[N]) {
-    unsigned m[N];
-    int total = 0;
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-        m[k] = __ballot_sync(0xffffffffu, want[k]);
-        total += __popc(m[k]);
-    }
-    int base = 0;
-    if (total > 0 && (threadIdx.x & 31) == 0) base = atomicAdd(counter, total);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    const unsigned lt = lanemask_lt();
-#pragma unroll
-    for (int k = 0; k < N; k++) {
-        slot[k] = want[k] ? base + __popc(m[k] & lt) : -1;
-        base += __popc(m[k]);
-    }
-}
-
-// Two warp-aggregated appends (counters ca and cb) whose atomics are both issued before
-// either result is read, so their round trips overlap.
-template <int N>
-__device__ __forceinline__ void warp_append_pair(int* ca, const bool (&wa)[N], int (&sa)[N], int* cb,
+__device__ __forceinline__ void warp_append_pair(unsigned long long* counter, const bool (&wa)[N], int (&sa)[N],
                                                  const bool (&wb)[N], int (&sb)[N]) {
     unsigned ma[N], mb[N];
     int ta = 0, tb = 0;
@@ -99,13 +78,11 @@ __device__ __forceinline__ void warp_append_pair(int* ca, const bool (&wa)[N], i
         ta += __popc(ma[k]);
         tb += __popc(mb[k]);
     }
-    int ba = 0, bb = 0;
-    if ((threadIdx.x & 31) == 0) {
-        if (ta > 0) ba = atomicAdd(ca, ta);
-        if (tb > 0) bb = atomicAdd(cb, tb);
-    }
-    ba = __shfl_sync(0xffffffffu, ba, 0);
-    bb = __shfl_sync(0xffffffffu, bb, 0);
+    unsigned long long base = 0;
+    if ((threadIdx.x & 31) == 0 && (ta | tb))
+        base = atomicAdd(counter, (unsigned long long)ta | ((unsigned long long)tb << 32));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    int ba = (int)(base & 0xffffffffu), bb = (int)(base >> 32);
     const unsigned lt = lanemask_lt();
 #pragma unroll
     for (int k = 0; k < N; k++) {
@@ -114,6 +91,14 @@ __device__ __forceinline__ void warp_append_pair(int* ca, const bool (&wa)[N], i
         ba += __popc(ma[k]);
         bb += __popc(mb[k]);
     }
+}
+
+// Rays in the queue consumed at `depth`, and shadow rays produced at it.
+__device__ __forceinline__ int ray_count(const FrameParams& p, int depth) {
+    return (int)(p.counters->depth[depth].appended & 0xffffffffu);
+}
+__device__ __forceinline__ int shadow_count(const FrameParams& p, int depth) {
+    return (int)(p.counters->depth[depth + 1].appended >> 32);
 }
 
 __device__ __forceinline__ void prefetch_l2(const void* ptr) {
@@ -216,7 +201,7 @@ __global__ void k_camera(FrameParams p, long long wave_first, int n) {
         p.L[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        p.counters->ray_count[0] = n;
+        p.counters->depth[0].appended = (unsigned long long)n;
         atomicAdd(&p.stats->rays_camera, (unsigned long long)n);
     }
 }
@@ -231,7 +216,7 @@ __global__ void k_wave_start(FrameParams p, int n) {
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
             p.L[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        p.counters->ray_count[0] = n;
+        p.counters->depth[0].appended = (unsigned long long)n;
         atomicAdd(&p.stats->rays_camera, (unsigned long long)n);
     }
 }
@@ -285,7 +270,7 @@ __device__ __forceinline__ int ray_sort_key(const GuideFrame& gf, float4 o, floa
 // unspecified.
 __global__ void __launch_bounds__(kRaySortBlock) k_ray_scatter(FrameParams p, int depth) {
     __shared__ int off[kRayBuckets], loc[kRayBuckets], wsum[kRaySortBlock / 32];
-    const int count = p.counters->ray_count[depth];
+    const int count = ray_count(p, depth);
     const PathQueue q = p.q[depth & 1];
     const int* cnt = p.ray_hist + 2 * depth * kRayBuckets;
     int* fill = p.ray_hist + (2 * depth + 1) * kRayBuckets;
@@ -326,7 +311,7 @@ template <int W, bool CNT, bool B, int Q>
 __global__ void k_extend(FrameParams p, int depth, long long wave_first) {
     extern __shared__ int2 stk[];
     __shared__ int s_class[8];  // the block's hits per material class
-    const int count = p.counters->ray_count[depth];
+    const int count = ray_count(p, depth);
     const PathQueue q = p.q[depth & 1];
     // NEE frames trace bounce rays from the BSDF-direct tMin and re-trace the rare ones whose
     // hit lies closer than the continuation's (see the file comment); at a path's last depth
@@ -361,7 +346,7 @@ __global__ void k_extend(FrameParams p, int depth, long long wave_first) {
             const int idle = 32 - __popc(busy);
             if (idle >= refill_idle) {  // refill_idle is in [1, 32]: an all-idle warp always fetches
                 int base = 0;
-                if (lane == 0) base = atomicAdd(&p.counters->work_extend[depth], idle);
+                if (lane == 0) base = atomicAdd(&p.counters->depth[depth].work_extend, idle);
                 base = __shfl_sync(0xffffffffu, base, 0);
                 if (base + idle >= count) more = false;
                 const int k = base + __popc(~busy & lanemask_lt());
@@ -424,20 +409,20 @@ __global__ void k_extend(FrameParams p, int depth, long long wave_first) {
     __syncthreads();
     // one atomic per class and block for the whole persistent loop
     if (p.shape.sort_materials && threadIdx.x < kMaterialClasses && s_class[threadIdx.x] > 0)
-        atomicAdd(&p.counters->sort_count[depth][threadIdx.x], s_class[threadIdx.x]);
+        atomicAdd(&p.counters->depth[depth].sort_count[threadIdx.x], s_class[threadIdx.x]);
     if (CNT) flush_work(work, &p.stats->extend_nodes, &p.stats->extend_prims);
 }
 
 constexpr int kSortItems = 4;  // queue entries per thread and chunk of the material sort
 __global__ void k_sort(FrameParams p, int depth) {
-    const int count = p.counters->ray_count[depth];
+    const int count = ray_count(p, depth);
     const PathQueue q = p.q[depth & 1];
     int off[kMaterialClasses];
     int acc = 0;
 #pragma unroll
     for (int c = 0; c < kMaterialClasses; c++) {
         off[c] = acc;
-        acc += p.counters->sort_count[depth][c];
+        acc += p.counters->depth[depth].sort_count[c];
     }
     // Slots are reserved per block and chunk of kSortItems x blockDim.x entries: warps add
     // their class counts into shared counters, then one global atomic per class and chunk
@@ -467,7 +452,7 @@ __global__ void k_sort(FrameParams p, int depth) {
         }
         __syncthreads();
         if (threadIdx.x < kMaterialClasses && s_cnt[threadIdx.x] > 0)
-            s_base[threadIdx.x] = atomicAdd(&p.counters->sort_fill[depth][threadIdx.x], s_cnt[threadIdx.x]);
+            s_base[threadIdx.x] = atomicAdd(&p.counters->depth[depth].sort_fill[threadIdx.x], s_cnt[threadIdx.x]);
         __syncthreads();
 #pragma unroll
         for (int j = 0; j < kSortItems; j++) {
@@ -620,14 +605,14 @@ __host__ __device__ constexpr int shade_class_regs(int cls) { return cls == kMic
 template <bool GUIDE, bool B, int CLS, int IPL, bool AHEAD = false>
 __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long long wave_first, long long gfirst) {
     constexpr int kType = CLS > 0 ? CLS - 1 : -1;  // the material type of a class kernel
-    int count = p.counters->ray_count[depth];
+    int count = ray_count(p, depth);
     int cls_first = 0;
     if constexpr (CLS >= 0) {  // the class's range of the sorted order
-        for (int c = 0; c < CLS; c++) cls_first += p.counters->sort_count[depth][c];
-        count = p.counters->sort_count[depth][CLS];
+        for (int c = 0; c < CLS; c++) cls_first += p.counters->depth[depth].sort_count[c];
+        count = p.counters->depth[depth].sort_count[CLS];
         if (count == 0) return;  // a class absent at this depth: no fetch, no atomics
     }
-    int* const work = CLS >= 0 ? &p.counters->work_class[depth][CLS < 0 ? 0 : CLS] : &p.counters->work_shade[depth];
+    int* const work = CLS >= 0 ? &p.counters->depth[depth].work_class[CLS < 0 ? 0 : CLS].v : &p.counters->depth[depth].work_shade;
     const PathQueue q = p.q[depth & 1];
     const PathQueue qn = p.q[(depth + 1) & 1];
     const bool last_frame = depth >= p.max_depth - 1;
@@ -647,18 +632,21 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
     // AHEAD: the chunk after next is claimed while a chunk shades (lane 0's atomic result,
     // read one chunk later), the next chunk's slots are loaded then too, and its queue records
     // are prefetched into L2 before this chunk's results are written
-    int claimed = 0, cur_base = 0, next_base = 0, cur_slot = -1;
+    // a warp's first chunk is its own by its index in the grid, the cursor serves the rest
+    const int first = ((int)(blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32 * IPL;
+    const int rest = (int)(gridDim.x * blockDim.x) * IPL;
+    int claimed = 0, cur_base = first, next_base = 0, cur_slot = -1;
     if (AHEAD) {
-        cur_base = warp_fetch(work);
-        next_base = warp_fetch(work);
+        if (rest < count) next_base = rest + warp_fetch(work);
+        else next_base = count;
         if (cur_base + lane < count) cur_slot = slot_of(cur_base + lane);
     }
     for (;;) {
-        const int base = AHEAD ? cur_base : warp_fetch(work, 32 * IPL);
+        const int base = cur_base;
         if (base >= count) break;
         int next_slot = -1;
         if (AHEAD) {
-            if (lane == 0) claimed = atomicAdd(work, 32);
+            if (lane == 0) claimed = next_base < count ? rest + atomicAdd(work, 32) : count;
             if (next_base + lane < count) next_slot = slot_of(next_base + lane);
         }
         bool cont_[IPL], shadow_[IPL];
@@ -874,11 +862,7 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
             prefetch_l2(q.rng + next_slot);
         }
         int cslot[IPL], sslot[IPL];
-        if (AHEAD)
-            warp_append_pair<IPL>(&p.counters->ray_count[depth + 1], cont_, cslot, &p.counters->shadow_count[depth],
-                                  shadow_, sslot);
-        else
-            warp_append_n<IPL>(&p.counters->ray_count[depth + 1], cont_, cslot);
+        warp_append_pair<IPL>(&p.counters->depth[depth + 1].appended, cont_, cslot, shadow_, sslot);
 #pragma unroll
         for (int item = 0; item < IPL; item++) {
             if (!cont_[item]) continue;
@@ -893,7 +877,6 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
                 atomicAdd(&rhist[key], 1);
             }
         }
-        if (!AHEAD) warp_append_n<IPL>(&p.counters->shadow_count[depth], shadow_, sslot);
 #pragma unroll
         for (int item = 0; item < IPL; item++) {
             if (!shadow_[item]) continue;
@@ -906,6 +889,8 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
             cur_base = next_base;
             next_base = __shfl_sync(0xffffffffu, claimed, 0);
             cur_slot = next_slot;
+        } else {
+            cur_base = rest < count ? rest + warp_fetch(work, 32 * IPL) : count;
         }
     }
     if (!B && rsort) {
@@ -949,7 +934,7 @@ __global__ void __maxnreg__(shade_class_regs(CLS)) k_shade_class(FrameParams p, 
 template <int W, bool CNT, bool B, int Q>
 __global__ void k_shadow(FrameParams p, int depth, long long wave_first, long long gfirst) {
     extern __shared__ int2 stk[];
-    const int count = p.counters->shadow_count[depth];
+    const int count = shadow_count(p, depth);
     const int lane = threadIdx.x & 31;
     const int refill_idle = p.shape.refill_idle;
     const bool spec = (p.shape.speculate & kSpeculateShadow) != 0;
@@ -967,14 +952,14 @@ __global__ void k_shadow(FrameParams p, int depth, long long wave_first, long lo
     Hit h{0.f, 0.f, 0.f, kMissPrim};  // unused by any-hit queries
     SceneDevice scb;
     if (B) scb = p.sc;
-    bool more = true;  // warp-uniform
+    bool more = true;  // warp-uniform: the queue may hold rays not yet taken
     for (;;) {
         if (more) {
             const unsigned busy = __ballot_sync(0xffffffffu, slot >= 0);
             const int idle = 32 - __popc(busy);
             if (idle >= refill_idle) {
                 int base = 0;
-                if (lane == 0) base = atomicAdd(&p.counters->work_shadow[depth], idle);
+                if (lane == 0) base = atomicAdd(&p.counters->depth[depth].work_shadow, idle);
                 base = __shfl_sync(0xffffffffu, base, 0);
                 if (base + idle >= count) more = false;
                 const int k = base + __popc(~busy & lanemask_lt());
@@ -1064,7 +1049,7 @@ __device__ __forceinline__ float* guide_activate_row(uint32_t* sx, int lane) {
 template <bool B>
 __global__ void __launch_bounds__(32 * kInferWarps, 2) k_guide_infer(FrameParams p, int depth) {
     extern __shared__ __align__(16) uint32_t ism[];
-    const int count = p.counters->ray_count[depth];
+    const int count = ray_count(p, depth);
     const int groups = (count + 31) / 32;
     if (blockIdx.x * kInferWarps >= groups) return;  // no rays for this block: skip the weight copy
     uint32_t* sw = ism;
@@ -1136,7 +1121,7 @@ __global__ void __launch_bounds__(32 * kInferWarps, 2) k_guide_infer(FrameParams
 __global__ void __launch_bounds__(kTcThreads, 2) k_guide_infer_tc(FrameParams p, int depth) {
     extern __shared__ __align__(1024) uint8_t tsm[];
     TcSmem& s = *reinterpret_cast<TcSmem*>(tsm);
-    const int count = p.counters->ray_count[depth];
+    const int count = ray_count(p, depth);
     const int tiles = (count + kTcThreads - 1) / kTcThreads;
     if ((int)blockIdx.x >= tiles) return;  // no work: skip the setup and the TMEM allocation
     const uint32_t tmem = tc_setup(s, p.gwpack, p.gwpack + kPackWords);
@@ -1323,6 +1308,28 @@ cudaError_t enqueue_class_shades(const FrameParams& p, int d, long long wave_fir
     return cudaSuccess;
 }
 
+using ExtendKernel = void (*)(FrameParams, int, long long);
+using ShadowKernel = void (*)(FrameParams, int, long long, long long);
+// The traversal kernels for the scene's node format and triangle test.
+template <int W, bool CNT, bool B>
+ExtendKernel extend_kernel(const SceneDevice& sc) {
+    if (sc.watertight) return k_extend<W, CNT, B, 2>;
+    return W >= 4 && sc.node_q ? k_extend<W, CNT, B, (W >= 4 ? 1 : 0)> : k_extend<W, CNT, B, 0>;
+}
+template <int W, bool CNT, bool B>
+ShadowKernel shadow_kernel(const SceneDevice& sc) {
+    if (sc.watertight) return k_shadow<W, CNT, B, 2>;
+    return W >= 4 && sc.node_q ? k_shadow<W, CNT, B, (W >= 4 ? 1 : 0)> : k_shadow<W, CNT, B, 0>;
+}
+
+// Blocks of a persistent grid: shape.blocks_per_sm per SM, at most what stays resident.
+cudaError_t resident_grid(const void* kernel, int block, size_t smem, const FrameParams& p, int& grid) {
+    int per_sm = 0;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
+    grid = p.num_sms * std::max(1, std::min(per_sm, p.shape.blocks_per_sm));
+    return e;
+}
+
 template <int W, bool CNT, bool B>
 cudaError_t enqueue_waves(const FrameParams& p_in, const WaveRange* waves, int nwaves, cudaStream_t stream,
                           StageMarks* marks, const SideStream* side) {
@@ -1331,7 +1338,6 @@ cudaError_t enqueue_waves(const FrameParams& p_in, const WaveRange* waves, int n
     FrameParams p = p_in;
     const bool classes = p.shape.shade_kernel == kShadeClasses && p.shape.sort_materials && p.class_mask;
     p.cam_fused = p.shape.fuse_camera && !p.guide_mode && !classes && p.shape.shade_kernel != kShadeAll80 ? 1 : 0;
-    const int grid_e = p.num_sms * p.shape.blocks_per_sm;
     // shadow stage of depth d on the side stream: forked after the shade stage of d, joined
     // before the shade stage of d + 1 (which adds to the same path radiance after it); the
     // closest-hit stage of d + 1 runs beside it
@@ -1340,13 +1346,20 @@ cudaError_t enqueue_waves(const FrameParams& p_in, const WaveRange* waves, int n
     const cudaStream_t sstream = overlap ? side->stream : stream;
     const size_t smem_e = stack_bytes(p.stack_depth, p.shape.block_extend);
     const size_t smem_s = stack_bytes(p.stack_depth, p.shape.block_shadow);
+    // persistent traversal grids: at most as many blocks as stay resident
+    const ExtendKernel extend = extend_kernel<W, CNT, B>(p.sc);
+    const ShadowKernel shadow = shadow_kernel<W, CNT, B>(p.sc);
+    int grid_e = 0, grid_s = 0;
+    cudaError_t ge = resident_grid((const void*)extend, p.shape.block_extend, smem_e, p, grid_e);
+    if (ge == cudaSuccess) ge = resident_grid((const void*)shadow, p.shape.block_shadow, smem_s, p, grid_s);
+    if (ge != cudaSuccess) return ge;
     Marker mark{marks, stream};
     Marker smark{marks, sstream};  // the side stream's shadow stages
     for (int wv = 0; wv < nwaves; wv++) {
         const WaveRange& w = waves[wv];
         const int n = w.npaths;
         const long long wave_first = w.first_path;
-        cudaError_t e = cudaMemsetAsync(p.counters, 0, sizeof(WaveCounters), stream);
+        cudaError_t e = cudaMemsetAsync(p.counters, 0, (p.max_depth + 1) * sizeof(DepthCounters), stream);
         if (e != cudaSuccess) return e;
         const bool sort_rays = !B && p.shape.sort_rays;
         if (sort_rays && (e = cudaMemsetAsync(p.ray_hist, 0, 2 * p.max_depth * kRayBuckets * sizeof(int), stream)))
@@ -1365,14 +1378,7 @@ cudaError_t enqueue_waves(const FrameParams& p_in, const WaveRange* waves, int n
                 k_ray_scatter<<<p.num_sms * 4, kRaySortBlock, 0, stream>>>(p, d);
                 mark(kStageSort);
             }
-            if (p.sc.watertight) {
-                k_extend<W, CNT, B, 2><<<grid_e, p.shape.block_extend, smem_e, stream>>>(p, d, wave_first);
-            } else if constexpr (W >= 4) {
-                if (p.sc.node_q) k_extend<W, CNT, B, 1><<<grid_e, p.shape.block_extend, smem_e, stream>>>(p, d, wave_first);
-                else k_extend<W, CNT, B, 0><<<grid_e, p.shape.block_extend, smem_e, stream>>>(p, d, wave_first);
-            } else {
-                k_extend<W, CNT, B, 0><<<grid_e, p.shape.block_extend, smem_e, stream>>>(p, d, wave_first);
-            }
+            extend<<<grid_e, p.shape.block_extend, smem_e, stream>>>(p, d, wave_first);
             mark(kStageExtend);
             if (p.shape.sort_materials) {
                 k_sort<<<std::min((n + 256 * kSortItems - 1) / (256 * kSortItems), p.num_sms * 8), 256, 0, stream>>>(
@@ -1410,15 +1416,7 @@ cudaError_t enqueue_waves(const FrameParams& p_in, const WaveRange* waves, int n
                     if ((e = cudaStreamWaitEvent(sstream, side->shaded[d], 0))) return e;
                     smark(-1);
                 }
-                if (p.sc.watertight)
-                    k_shadow<W, CNT, B, 2><<<grid_e, p.shape.block_shadow, smem_s, sstream>>>(p, d, wave_first,
-                                                                                            w.guided_first);
-                else if (W >= 4 && p.sc.node_q)
-                    k_shadow<W, CNT, B, (W >= 4 ? 1 : 0)><<<grid_e, p.shape.block_shadow, smem_s, sstream>>>(
-                        p, d, wave_first, w.guided_first);
-                else
-                    k_shadow<W, CNT, B, 0><<<grid_e, p.shape.block_shadow, smem_s, sstream>>>(p, d, wave_first,
-                                                                                            w.guided_first);
+                shadow<<<grid_s, p.shape.block_shadow, smem_s, sstream>>>(p, d, wave_first, w.guided_first);
                 if (overlap) {
                     if ((e = cudaEventRecord(side->shadowed[d], sstream))) return e;
                     smark(kStageShadow);

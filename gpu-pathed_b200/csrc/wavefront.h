@@ -30,16 +30,29 @@ struct ShadowQueue {
 
 constexpr int kMaxDepthLimit = 64;
 
-// Device counters of one wave (zeroed at wave start).
+// Device counters of one depth of a wave (zeroed at wave start). Every warp of a stage's grid
+// adds to the stage's cursor and to the queue lengths, and one L2 slice serves about 1.5 such
+// atomics per ns whatever addresses they name (measured on a B200: 1.45 per ns for one
+// counter, 1.3 for two 128 B apart, 1.6 for two 512 B apart, 2.9 for two 4 KB apart, 5.4 for four).
+// So each counter that every warp hits lies in its own 4 KB page, and the shade stage appends to
+// both of its queues with one atomic (three per 32 paths before, on counters 260 B apart). Frame times
+// before -> after, with grids capped at what stays resident: 1024x1024 spheres at 64 spp 25.92 ->
+// 25.73 ms, 1.31M-triangle mesh at 1080p and 32 spp 34.00 -> 33.66, Cornell box 400x400 at 1 spp 0.39 -> 0.36.
+constexpr int kCounterPage = 4096;
+struct alignas(kCounterPage) DepthCounters {
+    // queue lengths: low half, rays in the queue consumed at this depth; high half, shadow rays
+    // produced at the depth before (one 64-bit atomic appends to both)
+    unsigned long long appended;
+    alignas(kCounterPage) int work_extend;  // persistent work-fetch cursors
+    alignas(kCounterPage) int work_shade;
+    alignas(kCounterPage) int work_shadow;
+    struct alignas(1024) Cursor { int v; };
+    alignas(kCounterPage) Cursor work_class[8];  // fetch cursors of the per-class shade kernels
+    alignas(kCounterPage) int sort_count[8];     // per material class hit counts (sorted shading)
+    alignas(1024) int sort_fill[8];
+};
 struct WaveCounters {
-    int ray_count[kMaxDepthLimit + 1];     // rays in the queue consumed at depth d
-    int shadow_count[kMaxDepthLimit + 1];  // shadow rays produced at depth d
-    int work_extend[kMaxDepthLimit + 1];   // persistent work-fetch cursors
-    int work_shade[kMaxDepthLimit + 1];
-    int work_shadow[kMaxDepthLimit + 1];
-    int work_class[kMaxDepthLimit + 1][8];  // fetch cursors of the per-class shade kernels
-    int sort_count[kMaxDepthLimit + 1][8]; // per material class hit counts (sorted shading)
-    int sort_fill[kMaxDepthLimit + 1][8];
+    DepthCounters depth[kMaxDepthLimit + 1];
 };
 
 // Frame-wide device statistics (not reset per wave).
