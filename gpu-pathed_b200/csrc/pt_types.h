@@ -140,6 +140,23 @@ struct SceneDevice {
     int watertight;            // 1: triangle leaf entries hold p0, p1, p2 and take the watertight test
 };
 
+// Traversal stacks of a launch (LaneStack in dev_trace.cuh): entries per lane in shared memory,
+// and the global memory behind them, [entry][thread of the grid].
+struct StackShape {
+    int shared;        // entries in shared memory
+    int cap;           // entries a query may use (the tree's need; less only under the test hook)
+    int spill_stride;  // threads `spill` has room for
+    int pad;
+    void* spill;       // cap - shared entries per thread (null when the need fits in shared memory)
+};
+// What a tree may need: at most width - 1 children left behind per level.
+PT_HD int stack_need(int width, int depth) { return (width - 1) * (depth + 1); }
+// Entries per lane in shared memory. 12 of 8 bytes take 106 KB at the 1024 threads per SM that 64
+// registers leave resident, so the L1 keeps about 96 KB for nodes and leaf entries; few lanes go
+// deeper. Frame ms with 6 / 8 / 11 / 12 / 16 entries: mesh 28.6 / 27.9 / 27.7 / 27.6 / 27.9, slit room 77.5 / 76.4 /
+// 75.7 / 75.7 / 75.9, guided slit room (shorter, latency-bound launches) 4.42 / 4.34 / 4.31 / 4.30 / 4.70.
+constexpr int kStackShared = 12;
+
 // Ray-query kinds and their [tMin, tMax] conventions (src/renderers/path_tracer.cu):
 //   camera rays tMin 0 (:154), continuation 1e-3 (:177), BSDF-direct 1e-4 (:51),
 //   shadow [1e-4, distance - 2e-4] (:104-108).

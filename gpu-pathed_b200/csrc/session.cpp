@@ -826,8 +826,30 @@ int Session::upload_scene() {
         if (qf) return fail(PT_ERR_SCENE, "a BVH node could not be quantized conservatively");
     }
     if (batch_mode() && (r = upload_batch())) return r;
+    if ((r = ensure_stacks())) return r;
     scene_dirty_ = false;
     return upload_materials();
+}
+
+// Stacks of `threads` lanes for the tree on the device, their global part in `spill`.
+StackShape Session::stack_shape(const DevBuf& spill, int threads) const {
+    StackShape st{};
+    const int need = stack_need(bvh_.width, bvh_.depth);
+    st.shared = std::min(need, kStackShared);
+    st.cap = test_stack_cap_ > 0 ? std::min(test_stack_cap_, need) : need;
+    st.spill_stride = threads;
+    st.spill = need > st.shared ? spill.p : nullptr;
+    return st;
+}
+
+int Session::ensure_stacks() {
+    const int need = stack_need(bvh_.width, bvh_.depth);
+    if (need <= kStackShared) return PT_OK;
+    int r;
+    const size_t deep = (size_t)(need - kStackShared), lanes = (size_t)num_sms_ * kSmThreads;
+    if ((r = check_cuda(d_spill_.alloc(deep * lanes * sizeof(int2)), "traversal stacks"))) return r;
+    if ((r = check_cuda(d_shadow_spill_.alloc(deep * lanes * sizeof(int)), "traversal stacks"))) return r;
+    return check_cuda(d_query_spill_.alloc(deep * kStaticTraceMaxRays * sizeof(int2)), "traversal stacks");
 }
 
 SceneDevice Session::scene_view() const {
@@ -943,10 +965,10 @@ int Session::render_async(int spp) {
     if ((r = ensure_frame_buffers(spp))) return r;
     std::string err;
     if (!batch && !make_camera(camspec_, w_, h_, cam_, err)) return fail(PT_ERR_ARG, err);
-    const int stack_depth = bvh_.depth + 1;
     const int maxb = std::max(shape_.block_extend, shape_.block_shadow);
-    const size_t smem = stack_bytes(stack_depth, maxb);
-    if (smem > max_smem_) return fail(PT_ERR_SCENE, "BVH too deep for the traversal stack in shared memory");
+    if (level_bytes(bvh_.depth + 1, maxb) > max_smem_)
+        return fail(PT_ERR_SCENE, "BVH too deep for the traversal stack in shared memory");
+    const size_t smem = (size_t)kStackShared * maxb * sizeof(int2);
     if (smem > smem_configured_) {
         if ((r = check_cuda(configure_traversal_smem(smem), "shared memory configuration"))) return r;
         smem_configured_ = smem;
@@ -994,7 +1016,8 @@ int Session::render_async(int spp) {
         p.batch_pixel_base = d_batch_pixel_base_.as<long long>();
         p.num_scenes = (int)batch_.size();
     }
-    p.stack_depth = stack_entries();
+    p.stack = stack_shape(d_spill_, num_sms_ * kSmThreads);
+    p.shadow_stack = stack_shape(d_shadow_spill_, num_sms_ * kSmThreads);
     p.mma_test_polls = test_mma_polls_;
     p.num_sms = num_sms_;
     p.count_work = work_counters_;
@@ -1579,7 +1602,9 @@ int Session::hit_test(int x, int y, int* mat) {
     if ((r = check_cuda(d_scratch_.alloc(64), "scratch"))) return r;
     int* dm = d_scratch_.as<int>();
     if ((r = check_cuda(cudaMemsetAsync(dm, 0, 8, stream_), "memset"))) return r;
-    if ((r = check_cuda(enqueue_hit_test(scene_view(), cam_, bvh_.depth + 1, x, y, dm, dm + 1, stream_), "hit test")))
+    StackShape stack = stack_shape(d_spill_, 32);  // one query: all of its entries in shared memory
+    stack.shared = stack.cap = stack_need(bvh_.width, bvh_.depth);
+    if ((r = check_cuda(enqueue_hit_test(scene_view(), cam_, stack, x, y, dm, dm + 1, stream_), "hit test")))
         return r;
     int res[2];
     if ((r = check_cuda(cudaMemcpyAsync(res, dm, 8, cudaMemcpyDeviceToHost, stream_), "hit test readback"))) return r;
@@ -1601,13 +1626,13 @@ int Session::trace_rays(const float* o, const float* d, const float* tmin, const
     if (in_flight_ && (r = wait(nullptr))) return r;
     if (scene_dirty_ && (r = upload_scene())) return r;
     if (mats_dirty_ && (r = upload_materials())) return r;
-    const int sd = stack_entries();
-    if (stack_bytes(sd, 128) > (size_t)kMaxStackBytesDefault)
+    const StackShape sd = stack_shape(d_spill_, num_sms_ * kSmThreads);
+    if (level_bytes(std::min(sd.cap, bvh_.depth + 1), 128) > (size_t)kMaxStackBytesDefault)
         return fail(PT_ERR_SCENE, "BVH too deep for the traversal stack in shared memory");
     if (device_ptrs) {
         if ((r = check_cuda(d_scratch_.alloc(64), "scratch"))) return r;
         int* of = d_scratch_.as<int>();
-        if ((r = check_cuda(cudaMemsetAsync(of, 0, 4, stream_), "memset"))) return r;
+        if ((r = check_cuda(cudaMemsetAsync(of, 0, 8, stream_), "memset"))) return r;  // the flag and the cursor
         if ((r = check_cuda(enqueue_trace_rays(scene_view(), sd, o, d, tmin, tmax, n, pty, pid, mid, t, bary, of, stream_),
                             "trace rays")))
             return r;
@@ -1637,7 +1662,7 @@ int Session::trace_rays(const float* o, const float* d, const float* tmin, const
     if ((r = check_cuda(cudaMemcpyAsync(dD, d, 12 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
     if ((r = check_cuda(cudaMemcpyAsync(dTmin, tmin, 4 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
     if ((r = check_cuda(cudaMemcpyAsync(dTmax, tmax, 4 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
-    if ((r = check_cuda(cudaMemsetAsync(dOf, 0, 4, st), "memset"))) return r;
+    if ((r = check_cuda(cudaMemsetAsync(dOf, 0, 8, st), "memset"))) return r;
     if ((r = check_cuda(enqueue_trace_rays(scene_view(), sd, dO, dD, dTmin, dTmax, n, dPt, dPid, dMid, dT,
                                            bary ? dB : nullptr, dOf, st),
                         "trace rays")))
@@ -1666,8 +1691,9 @@ int Session::trace_rays_static(const float* o, const float* d, const float* tmin
         return fail(PT_ERR_STATE,
                     "scene not resident on the device; make one allocating device call (render, trace, hit "
                     "test) after loading or editing the scene");
-    const int sd = bvh_.depth + 1;
-    if (stack_bytes(sd, 128) > (size_t)kMaxStackBytesDefault)
+    StackShape sd = stack_shape(d_query_spill_, kStaticTraceMaxRays);
+    sd.cap = stack_need(bvh_.width, bvh_.depth);
+    if (level_bytes(bvh_.depth + 1, 128) > (size_t)kMaxStackBytesDefault)
         return fail(PT_ERR_SCENE, "BVH too deep for the traversal stack in shared memory");
     int r;
     if ((r = check_cuda(cudaSetDevice(device_), "cudaSetDevice"))) return r;
@@ -1692,7 +1718,7 @@ int Session::occluded(const float* o, const float* d, const float* tmin, const f
     if (in_flight_ && (r = wait(nullptr))) return r;
     if (scene_dirty_ && (r = upload_scene())) return r;
     if (mats_dirty_ && (r = upload_materials())) return r;
-    const int sd = stack_entries();
+    const StackShape sd = stack_shape(d_spill_, num_sms_ * kSmThreads);
     const size_t N = (size_t)n;
     if ((r = check_cuda(d_scratch_.alloc(N * 4 * 9 + 256), "scratch"))) return r;
     float* dO = d_scratch_.as<float>();
@@ -1706,7 +1732,7 @@ int Session::occluded(const float* o, const float* d, const float* tmin, const f
     if ((r = check_cuda(cudaMemcpyAsync(dD, d, 12 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
     if ((r = check_cuda(cudaMemcpyAsync(dTmin, tmin, 4 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
     if ((r = check_cuda(cudaMemcpyAsync(dTmax, tmax, 4 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
-    if ((r = check_cuda(cudaMemsetAsync(dOf, 0, 4, st), "memset"))) return r;
+    if ((r = check_cuda(cudaMemsetAsync(dOf, 0, 8, st), "memset"))) return r;
     if ((r = check_cuda(enqueue_occluded(scene_view(), sd, dO, dD, dTmin, dTmax, n, dOcc, dOf, st), "occluded"))) return r;
     if ((r = check_cuda(cudaMemcpyAsync(occ, dOcc, 4 * N, cudaMemcpyDeviceToHost, st), "copy"))) return r;
     int hof = 0;

@@ -200,7 +200,7 @@ private:
     float stage_ms_[kNumStages] = {};
     int stage_launches_[kNumStages] = {};
     int last_wave_paths_ = 0;
-    size_t smem_configured_ = 48 * 1024;
+    size_t smem_configured_ = 40 * 1024;  // without opting in: 48 KB with the kernels' static part
     // per-frame constants (device) and their pinned staging copy
     DevBuf d_dyn_;
     FrameDyn* h_dyn_ = nullptr;
@@ -309,10 +309,11 @@ private:
     // non-blocking polls of the first wait of each tensor-core inference layer
     int test_stack_cap_ = 0;
     int test_mma_polls_ = 0;
-    int stack_entries() const {
-        const int sd = bvh_.depth + 1;
-        return test_stack_cap_ > 0 && test_stack_cap_ < sd ? test_stack_cap_ : sd;
-    }
+    // traversal stacks (dev_trace.cuh, LaneStack): the closest-hit stage and the queries on
+    // stream_, the shadow stage beside it, and the allocation-free queries on query_stream_
+    DevBuf d_spill_, d_shadow_spill_, d_query_spill_;
+    int ensure_stacks();
+    StackShape stack_shape(const DevBuf& spill, int threads) const;
 };
 
 }  // namespace pt

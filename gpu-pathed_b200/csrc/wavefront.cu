@@ -307,9 +307,14 @@ __global__ void __launch_bounds__(kRaySortBlock) k_ray_scatter(FrameParams p, in
 // terminated rays). With refill_idle = 32 a warp takes 32 new rays only after all of its
 // queries ended. With kSpeculateExtend set, traverse_round parks each lane's first leaf and
 // keeps descending while another lane of the warp still searches for one.
+// 64 registers keep 8 blocks of 128 threads resident; left to itself the compiler takes 76 (7 blocks;
+// mesh 28.4 ms against 27.6, slit room 79.1 against 75.7). Width 8 spills at 64.
+__host__ __device__ constexpr int traversal_regs(int width) { return width == 8 ? 80 : 64; }
+
 template <int W, bool CNT, bool B, int Q>
-__global__ void k_extend(FrameParams p, int depth, long long wave_first) {
+__global__ void __maxnreg__(traversal_regs(W)) k_extend(FrameParams p, int depth, long long wave_first) {
     extern __shared__ int2 stk[];
+    const LaneStack<false> st{stk + threadIdx.x, (int)blockDim.x, p.stack};
     __shared__ int s_class[8];  // the block's hits per material class
     const int count = ray_count(p, depth);
     const PathQueue q = p.q[depth & 1];
@@ -326,8 +331,6 @@ __global__ void k_extend(FrameParams p, int depth, long long wave_first) {
     if (threadIdx.x < 8) s_class[threadIdx.x] = 0;
     __syncthreads();
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&p.stats->rays_extend, (unsigned long long)count);
-    int2* const st = stk + threadIdx.x;
-    const int stride = blockDim.x;
     TraceWork work;
     // the lane's query; slot < 0: none (then alive is false as well)
     int slot = -1, cur = kEmptyChild, pend = kEmptyChild, sp = 0, of = 0;
@@ -376,8 +379,8 @@ __global__ void k_extend(FrameParams p, int depth, long long wave_first) {
         // with no query left after a fetch, the queue is exhausted (more is false)
         if (!__any_sync(0xffffffffu, alive)) break;
         const SceneDevice& sc = B ? scb : p.sc;
-        traverse_round<W, false, CNT>(sc.nodes, sc.prims, quant, spec, r, tmin, FLT_MAX, st, stride, p.stack_depth, h,
-                                      cur, pend, sp, alive, hit_any, of, &work, Q == 2);
+        traverse_round<W, false, CNT>(sc.nodes, sc.prims, quant, spec, r, tmin, FLT_MAX, st, h, cur, pend, sp, alive,
+                                      hit_any, of, &work, Q == 2);
         // a triangle at t = tMin is inside the continuation's range, a sphere is not (triangle.cu:34
         // accepts t >= tMin, sphere.cu:16,29 need t > tMin)
         if (slot >= 0 && !alive && retrace && !second && h.prim != kMissPrim &&
@@ -932,8 +935,9 @@ __global__ void __maxnreg__(shade_class_regs(CLS)) k_shade_class(FrameParams p, 
 }
 
 template <int W, bool CNT, bool B, int Q>
-__global__ void k_shadow(FrameParams p, int depth, long long wave_first, long long gfirst) {
-    extern __shared__ int2 stk[];
+__global__ void __maxnreg__(traversal_regs(W)) k_shadow(FrameParams p, int depth, long long wave_first, long long gfirst) {
+    extern __shared__ int stk_any[];
+    const LaneStack<true> st{stk_any + threadIdx.x, (int)blockDim.x, p.shadow_stack};
     const int count = shadow_count(p, depth);
     const int lane = threadIdx.x & 31;
     const int refill_idle = p.shape.refill_idle;
@@ -941,8 +945,6 @@ __global__ void k_shadow(FrameParams p, int depth, long long wave_first, long lo
     const bool near = p.shape.shadow_near != 0;  // children nearest first
     const bool quant = W >= 4 && Q == 1;
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&p.stats->rays_shadow, (unsigned long long)count);
-    int2* const st = stk + threadIdx.x;
-    const int stride = blockDim.x;
     TraceWork work;
     // the lane's query, refilled as in k_extend; slot < 0: none
     int slot = -1, cur = kEmptyChild, pend = kEmptyChild, sp = 0, of = 0, tag = 0;
@@ -981,8 +983,8 @@ __global__ void k_shadow(FrameParams p, int depth, long long wave_first, long lo
         }
         if (!__any_sync(0xffffffffu, alive)) break;
         const SceneDevice& sc = B ? scb : p.sc;
-        traverse_round<W, true, CNT>(sc.nodes, sc.prims, quant, spec, r, kShadowTMin, tmax, st, stride, p.stack_depth,
-                                     h, cur, pend, sp, alive, occ, of, &work, Q == 2, near);
+        traverse_round<W, true, CNT>(sc.nodes, sc.prims, quant, spec, r, kShadowTMin, tmax, st, h, cur, pend, sp, alive,
+                                     occ, of, &work, Q == 2, near);
         if (slot >= 0 && !alive) {  // the query ended: occluded, or the stack ran empty
             const int i = slot;
             slot = -1;
@@ -1344,8 +1346,8 @@ cudaError_t enqueue_waves(const FrameParams& p_in, const WaveRange* waves, int n
     const bool concurrent = side && side->stream && p.shape.overlap_shadow;
     const bool overlap = concurrent && p.nee;
     const cudaStream_t sstream = overlap ? side->stream : stream;
-    const size_t smem_e = stack_bytes(p.stack_depth, p.shape.block_extend);
-    const size_t smem_s = stack_bytes(p.stack_depth, p.shape.block_shadow);
+    const size_t smem_e = stack_bytes(p.stack, p.shape.block_extend, sizeof(int2));
+    const size_t smem_s = stack_bytes(p.shadow_stack, p.shape.block_shadow, sizeof(int));
     // persistent traversal grids: at most as many blocks as stay resident
     const ExtendKernel extend = extend_kernel<W, CNT, B>(p.sc);
     const ShadowKernel shadow = shadow_kernel<W, CNT, B>(p.sc);
@@ -1467,26 +1469,30 @@ __device__ __forceinline__ V hit_normal_rn(const SceneDevice& sc, V o, V d, cons
 template <int W>
 __global__ void k_normals(FrameParams p, int first_pixel, int npix) {
     extern __shared__ int2 stk[];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < npix;  // every lane enters the warp-synchronous traversal
-    const int pixel = first_pixel + (valid ? i : 0);
-    const int row = pixel / p.width, col = pixel - row * p.width;
-    V o, d;
-    camera_ray(p.dyn->cam, row, col, 0.5f, 0.5f, o, d);
-    const RayPre r = make_raypre(o, d);
-    Hit h;
-    int of = 0;
-    traverse<W, false>(p.sc, r, kCameraTMin, FLT_MAX, valid, stk + threadIdx.x, blockDim.x, p.stack_depth, h, of);
+    const LaneStack<false> st{stk + threadIdx.x, (int)blockDim.x, p.stack};
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&p.stats->rays_camera, (unsigned long long)npix);
-    if (!valid) return;
-    if (of) atomicOr(&p.stats->error, 1);
-    float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (h.prim != kMissPrim) {
-        const V n = hit_normal_rn(p.sc, o, d, h);
-        out = make_float4(__fdiv_rn(__fadd_rn(n.x, 1.f), 2.f), __fdiv_rn(__fadd_rn(n.y, 1.f), 2.f),
-                          __fdiv_rn(__fadd_rn(n.z, 1.f), 2.f), 0.f);
+    // every lane of a block enters the warp-synchronous traversal
+    for (int base = blockIdx.x * blockDim.x; base < npix; base += gridDim.x * blockDim.x) {
+        const int i = base + threadIdx.x;
+        const bool valid = i < npix;
+        const int pixel = first_pixel + (valid ? i : 0);
+        const int row = pixel / p.width, col = pixel - row * p.width;
+        V o, d;
+        camera_ray(p.dyn->cam, row, col, 0.5f, 0.5f, o, d);
+        const RayPre r = make_raypre(o, d);
+        Hit h;
+        int of = 0;
+        traverse<W, false>(p.sc, r, kCameraTMin, FLT_MAX, valid, st, h, of);
+        if (!valid) continue;
+        if (of) atomicOr(&p.stats->error, 1);
+        float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (h.prim != kMissPrim) {
+            const V n = hit_normal_rn(p.sc, o, d, h);
+            out = make_float4(__fdiv_rn(__fadd_rn(n.x, 1.f), 2.f), __fdiv_rn(__fadd_rn(n.y, 1.f), 2.f),
+                              __fdiv_rn(__fadd_rn(n.z, 1.f), 2.f), 0.f);
+        }
+        p.L[i] = out;
     }
-    p.L[i] = out;
 }
 
 // Normals frame: waves of whole pixels, one pixel-centre ray each, then the accumulation.
@@ -1494,12 +1500,14 @@ template <int W>
 cudaError_t enqueue_normals_w(const FrameParams& p, cudaStream_t stream, StageMarks* marks) {
     const int npixels = p.width * p.height;
     const int bs = p.shape.block_extend;  // the stack size the session configured covers this block
-    const size_t smem = stack_bytes(p.stack_depth, bs);
+    const size_t smem = stack_bytes(p.stack, bs, sizeof(int2));
+    // a block per bs pixels, at most what the stacks' global part has room for
+    const int most = std::max(1, p.stack.spill_stride / bs);
     Marker mark{marks, stream};
     mark(-1);
     for (int first = 0; first < npixels; first += p.wave_pixels) {
         const int npix = npixels - first < p.wave_pixels ? npixels - first : p.wave_pixels;
-        k_normals<W><<<(npix + bs - 1) / bs, bs, smem, stream>>>(p, first, npix);
+        k_normals<W><<<std::min((npix + bs - 1) / bs, most), bs, smem, stream>>>(p, first, npix);
         mark(kStageExtend);
         k_accumulate<false><<<(npix + 127) / 128, 128, 0, stream>>>(p, first, npix, (long long)first);
         mark(kStageAccum);
@@ -1565,61 +1573,86 @@ cudaError_t set_smem_w(size_t bytes) {
     return cudaSuccess;
 }
 
-template <int W>
-__global__ void k_trace_rays(SceneDevice sc, int stack_depth, const float* __restrict__ o,
-                             const float* __restrict__ d, const float* __restrict__ tmin,
-                             const float* __restrict__ tmax, int n, int* prim_type, int* prim_id, int* mat_id,
-                             float* t, float* bary, int* overflow) {
+// Caller-provided queries, persistent: a warp's first 32 rays are its own by its index in the
+// grid, later ones come from a cursor, taken (as in the closest-hit stage) whenever half the
+// warp's lanes are idle. flags[0]: the overflow flag, flags[1]: the cursor.
+constexpr int kQueryBlock = 128;
+constexpr int kQueryRefill = 16;
+struct QueryRays {
+    const float *o, *d, *tmin, *tmax;
+    int n;
+};
+struct QueryHits {  // closest hit: the five arrays (bary may be null); any hit: occluded
+    int *prim_type, *prim_id, *mat_id;
+    float *t, *bary;
+    int* occluded;
+};
+template <int W, bool ANY>
+__global__ void __launch_bounds__(kQueryBlock) k_query(SceneDevice sc, StackShape shape, QueryRays rays, QueryHits out, int* flags) {
     extern __shared__ int2 stk[];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < n;  // every lane enters the warp-synchronous traversal
-    const int j = valid ? i : 0;
-    const RayPre r = make_raypre(mkv(o[3 * j], o[3 * j + 1], o[3 * j + 2]), mkv(d[3 * j], d[3 * j + 1], d[3 * j + 2]));
-    Hit h;
-    int of = 0;
-    traverse<W, false>(sc, r, tmin[j], tmax[j], valid, stk + threadIdx.x, blockDim.x, stack_depth, h, of);
-    if (!valid) return;
-    if (of) atomicOr(overflow, 1);
-    if (h.prim == kMissPrim) {
-        prim_type[i] = -1;
-        prim_id[i] = -1;
-        mat_id[i] = -1;
-        t[i] = 0.f;
-        if (bary) { bary[2 * i] = 0.f; bary[2 * i + 1] = 0.f; }
-    } else if (h.prim >= 0) {
-        prim_type[i] = kTriangle;
-        prim_id[i] = h.prim;
-        mat_id[i] = sc.tri_mat[h.prim];
-        t[i] = h.t;
-        if (bary) { bary[2 * i] = h.b1; bary[2 * i + 1] = h.b2; }
-    } else {
-        prim_type[i] = kSphere;
-        prim_id[i] = ~h.prim;
-        mat_id[i] = sc.sph_mat[~h.prim];
-        t[i] = h.t;
-        if (bary) { bary[2 * i] = 0.f; bary[2 * i + 1] = 0.f; }
+    using Stack = LaneStack<ANY>;
+    const Stack st{reinterpret_cast<typename Stack::Entry*>(stk) + threadIdx.x, (int)blockDim.x, shape};
+    const bool quant = W >= 4 && sc.node_q != 0, wt = sc.watertight != 0;
+    const int lane = threadIdx.x & 31;
+    const int rest = gridDim.x * blockDim.x;  // first ray the cursor serves
+    int i = blockIdx.x * blockDim.x + threadIdx.x, cur = kEmptyChild, pend = kEmptyChild, sp = 0, of = 0;
+    bool alive = false, occ = false, first = true, more = true;
+    float tmin = 0.f, tmax = 0.f;
+    RayPre r = make_raypre(V{0.f, 0.f, 0.f}, V{0.f, 0.f, 1.f});
+    Hit h{0.f, 0.f, 0.f, kMissPrim};
+    for (;;) {
+        if (more) {
+            const unsigned idle = __ballot_sync(0xffffffffu, !alive);
+            if (__popc(idle) >= kQueryRefill) {
+                if (!first) {
+                    int base = 0;
+                    if (lane == 0) base = atomicAdd(flags + 1, __popc(idle));
+                    base = rest + __shfl_sync(0xffffffffu, base, 0);
+                    if (!alive) i = base + __popc(idle & lanemask_lt());
+                    more = base + __popc(idle) < rays.n;
+                } else {
+                    more = rest < rays.n;
+                }
+                first = false;
+                if (!alive && i < rays.n) {
+                    r = make_raypre(mkv(rays.o[3 * (size_t)i], rays.o[3 * (size_t)i + 1], rays.o[3 * (size_t)i + 2]),
+                                    mkv(rays.d[3 * (size_t)i], rays.d[3 * (size_t)i + 1], rays.d[3 * (size_t)i + 2]));
+                    tmin = rays.tmin[i];
+                    tmax = rays.tmax[i];
+                    h = Hit{tmax, 0.f, 0.f, kMissPrim};
+                    cur = sc.root;
+                    pend = kEmptyChild;
+                    sp = 0;
+                    of = 0;
+                    occ = false;
+                    alive = true;
+                }
+            }
+        }
+        if (!__any_sync(0xffffffffu, alive)) break;
+        const bool was = alive;
+        traverse_round<W, ANY, false>(sc.nodes, sc.prims, quant, false, r, tmin, tmax, st, h, cur, pend, sp, alive, occ,
+                                      of, nullptr, wt);
+        if (!was || alive) continue;
+        if (of) atomicOr(flags, 1);
+        if (ANY) {
+            out.occluded[i] = occ ? 1 : 0;
+        } else {
+            const bool hit = h.prim != kMissPrim, tri = hit && h.prim >= 0;
+            out.prim_type[i] = !hit ? -1 : tri ? kTriangle : kSphere;
+            out.prim_id[i] = !hit ? -1 : tri ? h.prim : ~h.prim;
+            out.mat_id[i] = !hit ? -1 : tri ? sc.tri_mat[h.prim] : sc.sph_mat[~h.prim];
+            out.t[i] = hit ? h.t : 0.f;
+            if (out.bary) {
+                out.bary[2 * (size_t)i] = tri ? h.b1 : 0.f;
+                out.bary[2 * (size_t)i + 1] = tri ? h.b2 : 0.f;
+            }
+        }
     }
 }
 
 template <int W>
-__global__ void k_occluded(SceneDevice sc, int stack_depth, const float* __restrict__ o,
-                           const float* __restrict__ d, const float* __restrict__ tmin,
-                           const float* __restrict__ tmax, int n, int* occluded, int* overflow) {
-    extern __shared__ int2 stk[];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool valid = i < n;
-    const int j = valid ? i : 0;
-    const RayPre r = make_raypre(mkv(o[3 * j], o[3 * j + 1], o[3 * j + 2]), mkv(d[3 * j], d[3 * j + 1], d[3 * j + 2]));
-    Hit h;
-    int of = 0;
-    const bool occ = traverse<W, true>(sc, r, tmin[j], tmax[j], valid, stk + threadIdx.x, blockDim.x, stack_depth, h, of);
-    if (!valid) return;
-    occluded[i] = occ ? 1 : 0;
-    if (of) atomicOr(overflow, 1);
-}
-
-template <int W>
-__global__ void k_hit_test(SceneDevice sc, CameraParams cam, int stack_depth, int x, int y, int* out, int* overflow) {
+__global__ void k_hit_test(SceneDevice sc, CameraParams cam, StackShape shape, int x, int y, int* out, int* overflow) {
     extern __shared__ int2 stk[];
     V o, d;
     camera_ray(cam, y, x, 0.5f, 0.5f, o, d);
@@ -1627,7 +1660,7 @@ __global__ void k_hit_test(SceneDevice sc, CameraParams cam, int stack_depth, in
     Hit h;
     int of = 0;
     // the whole warp enters the traversal; lane 0 carries the query and owns the stack
-    traverse<W, false>(sc, r, 0.f, FLT_MAX, threadIdx.x == 0, stk, 1, stack_depth, h, of);
+    traverse<W, false>(sc, r, 0.f, FLT_MAX, threadIdx.x == 0, LaneStack<false>{stk, 1, shape}, h, of);
     if (threadIdx.x != 0) return;
     if (of) atomicOr(overflow, 1);
     if (h.prim == kMissPrim) *out = -1;
@@ -1688,36 +1721,46 @@ cudaError_t configure_traversal_smem(size_t bytes) {
     return set_smem_w<8>(bytes);
 }
 
-cudaError_t enqueue_trace_rays(const SceneDevice& sc, int stack_depth, const float* o, const float* d,
+namespace {
+template <bool ANY>
+cudaError_t enqueue_query(const SceneDevice& sc, const StackShape& stack, const QueryRays& rays, const QueryHits& out,
+                          int* flags, cudaStream_t stream) {
+    if (rays.n <= 0) return cudaSuccess;
+    const void* kernel = sc.bvh_width == 2   ? (const void*)k_query<2, ANY>
+                         : sc.bvh_width == 4 ? (const void*)k_query<4, ANY>
+                         : sc.bvh_width == 8 ? (const void*)k_query<8, ANY>
+                                             : nullptr;
+    if (!kernel) return cudaErrorInvalidValue;
+    const size_t smem = stack_bytes(stack, kQueryBlock, ANY ? sizeof(int) : sizeof(int2));
+    // a block per kQueryBlock rays, at most what stays resident and what the stacks' global part has room for
+    int per_sm = 0, dev = 0, sms = 0;
+    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kQueryBlock, smem);
+    if (e != cudaSuccess || (e = cudaGetDevice(&dev)) != cudaSuccess ||
+        (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return e;
+    const int need = (int)(((long long)rays.n + kQueryBlock - 1) / kQueryBlock);
+    const int grid = std::max(1, std::min({need, per_sm * sms, stack.spill_stride / kQueryBlock}));
+    SceneDevice a0 = sc;
+    StackShape a1 = stack;
+    QueryRays a2 = rays;
+    QueryHits a3 = out;
+    void* args[] = {&a0, &a1, &a2, &a3, &flags};
+    return cudaLaunchKernel(kernel, dim3(grid), dim3(kQueryBlock), args, smem, stream);
+}
+}  // namespace
+
+cudaError_t enqueue_trace_rays(const SceneDevice& sc, const StackShape& stack, const float* o, const float* d,
                                const float* tmin, const float* tmax, int n, int* prim_type, int* prim_id,
-                               int* mat_id, float* t, float* bary, int* overflow, cudaStream_t stream) {
-    if (n <= 0) return cudaSuccess;
-    const int bs = 128;
-    const size_t smem = stack_bytes(stack_depth, bs);
-    const int grid = (n + bs - 1) / bs;
-    switch (sc.bvh_width) {
-        case 2: k_trace_rays<2><<<grid, bs, smem, stream>>>(sc, stack_depth, o, d, tmin, tmax, n, prim_type, prim_id, mat_id, t, bary, overflow); break;
-        case 4: k_trace_rays<4><<<grid, bs, smem, stream>>>(sc, stack_depth, o, d, tmin, tmax, n, prim_type, prim_id, mat_id, t, bary, overflow); break;
-        case 8: k_trace_rays<8><<<grid, bs, smem, stream>>>(sc, stack_depth, o, d, tmin, tmax, n, prim_type, prim_id, mat_id, t, bary, overflow); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+                               int* mat_id, float* t, float* bary, int* flags, cudaStream_t stream) {
+    return enqueue_query<false>(sc, stack, QueryRays{o, d, tmin, tmax, n},
+                                QueryHits{prim_type, prim_id, mat_id, t, bary, nullptr}, flags, stream);
 }
 
-cudaError_t enqueue_occluded(const SceneDevice& sc, int stack_depth, const float* o, const float* d,
-                             const float* tmin, const float* tmax, int n, int* occluded, int* overflow,
+cudaError_t enqueue_occluded(const SceneDevice& sc, const StackShape& stack, const float* o, const float* d,
+                             const float* tmin, const float* tmax, int n, int* occluded, int* flags,
                              cudaStream_t stream) {
-    if (n <= 0) return cudaSuccess;
-    const int bs = 128;
-    const size_t smem = stack_bytes(stack_depth, bs);
-    const int grid = (n + bs - 1) / bs;
-    switch (sc.bvh_width) {
-        case 2: k_occluded<2><<<grid, bs, smem, stream>>>(sc, stack_depth, o, d, tmin, tmax, n, occluded, overflow); break;
-        case 4: k_occluded<4><<<grid, bs, smem, stream>>>(sc, stack_depth, o, d, tmin, tmax, n, occluded, overflow); break;
-        case 8: k_occluded<8><<<grid, bs, smem, stream>>>(sc, stack_depth, o, d, tmin, tmax, n, occluded, overflow); break;
-        default: return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+    return enqueue_query<true>(sc, stack, QueryRays{o, d, tmin, tmax, n},
+                               QueryHits{nullptr, nullptr, nullptr, nullptr, nullptr, occluded}, flags, stream);
 }
 
 // ---- closest-hit queries without allocation ----------------------------------------------
@@ -1751,7 +1794,7 @@ cudaError_t static_scratch(float** out) {
 }
 }  // namespace
 
-cudaError_t trace_rays_static(const SceneDevice& sc, int stack_depth, const float* o, const float* d,
+cudaError_t trace_rays_static(const SceneDevice& sc, const StackShape& stack, const float* o, const float* d,
                               const float* tmin, const float* tmax, int n, int* prim_type, int* prim_id,
                               int* mat_id, float* t, float* bary, int* overflow, cudaStream_t stream) {
     if (n < 0 || n > kStaticTraceMaxRays) return cudaErrorInvalidValue;
@@ -1774,13 +1817,13 @@ cudaError_t trace_rays_static(const SceneDevice& sc, int stack_depth, const floa
     // into the caller's arrays lands after the call has returned.
     auto enqueue = [&]() -> cudaError_t {
         cudaError_t x;
-        if ((x = cudaMemsetAsync(sFlag, 0, sizeof(int), stream))) return x;
+        if ((x = cudaMemsetAsync(sFlag, 0, 2 * sizeof(int), stream))) return x;  // the flag and the cursor
         if (n == 0) return cudaSuccess;
         if ((x = cudaMemcpyAsync(sO, o, 3 * b, cudaMemcpyHostToDevice, stream))) return x;
         if ((x = cudaMemcpyAsync(sD, d, 3 * b, cudaMemcpyHostToDevice, stream))) return x;
         if ((x = cudaMemcpyAsync(sTmin, tmin, b, cudaMemcpyHostToDevice, stream))) return x;
         if ((x = cudaMemcpyAsync(sTmax, tmax, b, cudaMemcpyHostToDevice, stream))) return x;
-        if ((x = enqueue_trace_rays(sc, stack_depth, sO, sD, sTmin, sTmax, n, sType, sId, sMat, sT, sBary, sFlag,
+        if ((x = enqueue_trace_rays(sc, stack, sO, sD, sTmin, sTmax, n, sType, sId, sMat, sT, sBary, sFlag,
                                     stream)))
             return x;
         if ((x = cudaMemcpyAsync(prim_type, sType, b, cudaMemcpyDeviceToHost, stream))) return x;
@@ -1795,13 +1838,13 @@ cudaError_t trace_rays_static(const SceneDevice& sc, int stack_depth, const floa
     return e != cudaSuccess ? e : s;
 }
 
-cudaError_t enqueue_hit_test(const SceneDevice& sc, const CameraParams& cam, int stack_depth, int x, int y,
+cudaError_t enqueue_hit_test(const SceneDevice& sc, const CameraParams& cam, const StackShape& stack, int x, int y,
                              int* out_material, int* overflow, cudaStream_t stream) {
-    const size_t smem = stack_bytes(stack_depth, 1);
+    const size_t smem = stack_bytes(stack, 1, sizeof(int2));
     switch (sc.bvh_width) {
-        case 2: k_hit_test<2><<<1, 32, smem, stream>>>(sc, cam, stack_depth, x, y, out_material, overflow); break;
-        case 4: k_hit_test<4><<<1, 32, smem, stream>>>(sc, cam, stack_depth, x, y, out_material, overflow); break;
-        case 8: k_hit_test<8><<<1, 32, smem, stream>>>(sc, cam, stack_depth, x, y, out_material, overflow); break;
+        case 2: k_hit_test<2><<<1, 32, smem, stream>>>(sc, cam, stack, x, y, out_material, overflow); break;
+        case 4: k_hit_test<4><<<1, 32, smem, stream>>>(sc, cam, stack, x, y, out_material, overflow); break;
+        case 8: k_hit_test<8><<<1, 32, smem, stream>>>(sc, cam, stack, x, y, out_material, overflow); break;
         default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

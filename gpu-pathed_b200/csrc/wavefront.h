@@ -29,6 +29,7 @@ struct ShadowQueue {
 };
 
 constexpr int kMaxDepthLimit = 64;
+constexpr int kSmThreads = 2048;  // resident threads per SM, at most
 
 // Device counters of one depth of a wave (zeroed at wave start). Every warp of a stage's grid
 // adds to the stage's cursor and to the queue lengths, and one L2 slice serves about 1.5 such
@@ -203,7 +204,7 @@ struct FrameParams {
     int max_depth;
     int nee;
     int wave_pixels;         // pixels per wave
-    int stack_depth;         // traversal stack entries per thread
+    StackShape stack, shadow_stack;  // traversal stacks of the closest-hit and the shadow stage
     int num_sms;
     int count_work;          // 1: traversal kernels count nodes and leaf entries (slower)
     int renderer;            // 0 path tracer, 1 normals (one pixel-centre ray per pixel, spp 1)
@@ -256,18 +257,19 @@ cudaError_t configure_traversal_smem(size_t bytes);
 // Opt the guide inference kernel into its dynamic shared memory (weights + 8 warps x 32 rows).
 cudaError_t configure_guide_infer();
 
-// Closest-hit queries for caller-provided rays (parity entry). Arrays are device pointers.
-cudaError_t enqueue_trace_rays(const SceneDevice& sc, int stack_depth, const float* o, const float* d,
+// Closest-hit queries for caller-provided rays (parity entry). Arrays are device pointers; flags
+// holds two ints, zero at the launch: the overflow flag and the kernel's work cursor.
+cudaError_t enqueue_trace_rays(const SceneDevice& sc, const StackShape& stack, const float* o, const float* d,
                                const float* tmin, const float* tmax, int n, int* prim_type, int* prim_id,
-                               int* mat_id, float* t, float* bary, int* overflow, cudaStream_t stream);
+                               int* mat_id, float* t, float* bary, int* flags, cudaStream_t stream);
 
 // Any-hit queries for caller-provided rays: occluded[i] = 1 if something lies in [tmin, tmax].
-cudaError_t enqueue_occluded(const SceneDevice& sc, int stack_depth, const float* o, const float* d,
-                             const float* tmin, const float* tmax, int n, int* occluded, int* overflow,
+cudaError_t enqueue_occluded(const SceneDevice& sc, const StackShape& stack, const float* o, const float* d,
+                             const float* tmin, const float* tmax, int n, int* occluded, int* flags,
                              cudaStream_t stream);
 
 // One camera ray through the centre of pixel (x = col, y = row) (src/hit_test.cu:25-47).
-cudaError_t enqueue_hit_test(const SceneDevice& sc, const CameraParams& cam, int stack_depth, int x, int y,
+cudaError_t enqueue_hit_test(const SceneDevice& sc, const CameraParams& cam, const StackShape& stack, int x, int y,
                              int* out_material, int* overflow, cudaStream_t stream);
 
 // Closest-hit queries that allocate nothing: host rays in, host results out, staged through
@@ -275,7 +277,7 @@ cudaError_t enqueue_hit_test(const SceneDevice& sc, const CameraParams& cam, int
 // first call on a device looks the array's address up (cudaGetSymbolAddress) with that
 // device current. Returns cudaErrorInvalidValue for n outside [0, kStaticTraceMaxRays].
 constexpr int kStaticTraceMaxRays = 65536;
-cudaError_t trace_rays_static(const SceneDevice& sc, int stack_depth, const float* o, const float* d,
+cudaError_t trace_rays_static(const SceneDevice& sc, const StackShape& stack, const float* o, const float* d,
                               const float* tmin, const float* tmax, int n, int* prim_type, int* prim_id,
                               int* mat_id, float* t, float* bary, int* overflow, cudaStream_t stream);
 
@@ -283,7 +285,10 @@ cudaError_t trace_rays_static(const SceneDevice& sc, int stack_depth, const floa
 // `bytes` on the current device (probe.cu).
 cudaError_t measure_l2_read(size_t bytes, int reps, int trials, double* gbs, double* ms);
 
-// Size in bytes of the traversal stack per block for `threads` threads.
-inline size_t stack_bytes(int stack_depth, int threads) { return (size_t)stack_depth * threads * sizeof(int2); }
+// Shared memory of a block's traversal stacks (`entry` bytes per stack entry).
+inline size_t stack_bytes(const StackShape& st, int threads, size_t entry) { return (size_t)st.shared * threads * entry; }
+// Deepest tree a call takes: one 8-byte entry per level and thread must fit in the shared memory that the call may
+// ask for.
+inline size_t level_bytes(int levels, int threads) { return (size_t)levels * threads * sizeof(int2); }
 
 }  // namespace pt
