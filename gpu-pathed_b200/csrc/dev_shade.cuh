@@ -261,6 +261,17 @@ __device__ __forceinline__ V env_sample_dir(const EnvDevice& e, float xi1, float
     return wi;
 }
 
+// The lights of a path's scene: its range of the emitter list, its environment (where it lies: a
+// kernel parameter, or a batch's scene table) and the geometry arrays they index.
+struct SceneLights {
+    const SceneDevice& sc;
+    const LightRef* lights;
+    int num_lights;
+    const EnvDevice& env;
+    // emitters and the environment, each chosen with the same probability
+    __device__ __forceinline__ int choices() const { return num_lights + (env.present ? 1 : 0); }
+};
+
 // ---- Emitters (include/lights/sampler.h:20-183, surface_sample.h, core/measure.h) -------
 struct LightSample {
     V wi, normal;
@@ -273,14 +284,14 @@ __device__ __forceinline__ float tri_area(V p0, V p1, V p2) {
     return fabsf(length(c) / 2.f);
 }
 
-__device__ __forceinline__ LightSample sample_lights(const SceneDevice& sc, V p, float xi1, float xi2,
-                                                     float xi3) {
+__device__ __forceinline__ LightSample sample_lights(const SceneLights& sl, V p, float xi1, float xi2, float xi3) {
+    const SceneDevice& sc = sl.sc;
     LightSample ls;
-    const int n_choice = sc.num_lights + (sc.env.present ? 1 : 0);
+    const int n_choice = sl.choices();
     const int choice = (int)fminf((float)(n_choice - 1), (float)(int)floorf(xi1 * n_choice));
     const float choice_pdf = 1.f / n_choice;
-    if (choice < sc.num_lights) {
-        const LightRef lr = sc.lights[choice];
+    if (choice < sl.num_lights) {
+        const LightRef lr = sl.lights[choice];
         V point, normal;
         float area_pdf;
         int mat;
@@ -323,19 +334,20 @@ __device__ __forceinline__ LightSample sample_lights(const SceneDevice& sc, V p,
         if (m.type != kLambertian) ls.emitted = mkv(0.f);
     } else {
         float pdf;
-        const V w = env_sample_dir(sc.env, xi2, xi3, pdf);
+        const V w = env_sample_dir(sl.env, xi2, xi3, pdf);
         const V wi = normalized(w);
         ls.wi = wi;
         ls.normal = -wi;
         ls.distance = 1e16f;
         ls.pdf = pdf * choice_pdf;
-        ls.emitted = env_emit(sc.env, w);
+        ls.emitted = env_emit(sl.env, w);
     }
     return ls;
 }
 
-// Sampler::pdfSceneLights (sampler.h:89-125) for an emitting hit seen from `ref`.
-__device__ __forceinline__ float pdf_scene_light(const SceneDevice& sc, V ref, V point, V normal, int prim) {
+// Sampler::pdfSceneLights (sampler.h:89-125) for an emitting hit seen from `ref`, one of `n_choice` lights.
+__device__ __forceinline__ float pdf_scene_light(const SceneDevice& sc, int n_choice, V ref, V point, V normal,
+                                                 int prim) {
     float area_pdf;
     if (prim >= 0) {
         const V p0 = mkv(__ldg(sc.tri_p + 3 * prim + 0));
@@ -351,13 +363,12 @@ __device__ __forceinline__ float pdf_scene_light(const SceneDevice& sc, V ref, V
     const float dist = length(sd);
     const float proj = fmaxf(0.f, dot(normal, swo));
     const float sa = area_pdf * (dist * dist) / proj;
-    const int n_choice = sc.num_lights + (sc.env.present ? 1 : 0);
     return sa / n_choice;
 }
 // Sampler::pdfEnvironmentLight (sampler.h:127-140)
-__device__ __forceinline__ float pdf_env_light(const SceneDevice& sc, V w) {
-    if (!sc.env.present) return 0.f;
-    return env_pdf_dir(sc.env, w) * (1.f / (sc.num_lights + 1));
+__device__ __forceinline__ float pdf_env_light(const SceneLights& sl, V w) {
+    if (!sl.env.present) return 0.f;
+    return env_pdf_dir(sl.env, w) * (1.f / (sl.num_lights + 1));
 }
 // MIS::balanceWeight (include/math/mis.h:5-8)
 __device__ __forceinline__ float balance(float p1, float p2) { return p1 / (p1 + p2); }

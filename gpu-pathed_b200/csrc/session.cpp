@@ -719,7 +719,7 @@ int Session::set_launch(const pt_launch_config* c) {
     if (c->sort_rays) shape_.sort_rays = c->sort_rays == 1 ? 1 : 0;
     if (c->refill_idle) shape_.refill_idle = c->refill_idle;
     if (c->speculate) shape_.speculate = speculate_bits(c->speculate);
-    if (c->split_shade) shape_.shade_kernel = c->split_shade == 1 ? kShadeClasses : c->split_shade == 2 ? kShadeAll128 : kShadeAll80;
+    if (c->split_shade) shape_.shade_kernel = c->split_shade == 1 ? kShadeClasses : c->split_shade == 2 ? kShadeAllAhead : kShadeAllPlain;
     if (c->overlap_shadow) shape_.overlap_shadow = c->overlap_shadow == 1 ? 1 : 0;
     if (c->shadow_order) shape_.shadow_near = c->shadow_order == 1 ? 1 : 0;
     if (c->fuse_camera) shape_.fuse_camera = c->fuse_camera == 1 ? 1 : 0;
@@ -737,7 +737,7 @@ void Session::get_launch(pt_launch_config* c) const {
     c->sort_rays = shape_.sort_rays ? 1 : 2;
     c->refill_idle = shape_.refill_idle;
     c->speculate = speculate_code(shape_.speculate);
-    c->split_shade = shape_.shade_kernel == kShadeClasses ? 1 : shape_.shade_kernel == kShadeAll128 ? 2 : 3;
+    c->split_shade = shape_.shade_kernel == kShadeClasses ? 1 : shape_.shade_kernel == kShadeAllAhead ? 2 : 3;
     c->overlap_shadow = shape_.overlap_shadow ? 1 : 2;
     c->shadow_order = shape_.shadow_near ? 1 : 2;
     c->fuse_camera = shape_.fuse_camera ? 1 : 2;
@@ -1327,7 +1327,7 @@ int Session::autotune(int spp, const char* cache_path, pt_tune_result* out) {
         res.sort_rays = c.rays ? 1 : 2;
         res.speculate = speculate_code(c.spec);
         res.wave_paths = c.wave;
-        res.split_shade = c.split == kShadeClasses ? 1 : c.split == kShadeAll128 ? 2 : 3;
+        res.split_shade = c.split == kShadeClasses ? 1 : c.split == kShadeAllAhead ? 2 : 3;
         res.max_leaf = c.leaf;
         res.bvh_builder = c.builder == kGpuBvhPloc ? 2 : c.builder == kGpuBvhLbvh ? 1 : 0;
         res.shadow_order = c.near ? 1 : 2;
@@ -1428,9 +1428,9 @@ int Session::autotune(int spp, const char* cache_path, pt_tune_result* out) {
         c.sort = best.sort ? 0 : 1;
         if ((r = consider(c))) return r;
     }
-    if (!guiding_) {  // the plain shade stage: per-class kernels (sorted frames), one kernel at 128 or 80 registers
+    if (!guiding_) {  // the plain shade stage: per-class kernels (sorted frames), one kernel that fetches ahead or not
         const Cand base = best;
-        for (int k : {kShadeAll128, kShadeClasses, kShadeAll80})
+        for (int k : {kShadeAllAhead, kShadeClasses, kShadeAllPlain})
             if (k != base.split && (k != kShadeClasses || base.sort)) {
                 Cand c = base;
                 c.split = k;
@@ -1456,7 +1456,7 @@ int Session::autotune(int spp, const char* cache_path, pt_tune_result* out) {
         c.near = best.near ? 0 : 1;
         if ((r = consider(c))) return r;
     }
-    if (!guiding_) {  // camera rays computed where used (the 128-register shade kernel) or queued
+    if (!guiding_) {  // camera rays computed where used (the shade kernel that fetches ahead) or queued
         Cand c = best;
         c.fuse = best.fuse ? 0 : 1;
         if ((r = consider(c))) return r;

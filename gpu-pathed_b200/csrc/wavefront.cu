@@ -119,16 +119,16 @@ __device__ __forceinline__ int batch_find(const long long* base, int n, long lon
     return lo;
 }
 
-// The scene a path belongs to: in batched frames its root, emitter range and environment come
-// from the scene table (the geometry arrays are shared, with global primitive ids).
-__device__ __forceinline__ SceneDevice batch_scene_view(const FrameParams& p, int sid) {
-    SceneDevice sc = p.sc;
-    const BatchScene& b = p.batch[sid];
-    sc.root = b.root;
-    sc.lights = p.sc.lights + b.light_first;
-    sc.num_lights = b.num_lights;
-    sc.env = b.env;
-    return sc;
+// The lights of scene `sid`: in batched frames its emitter range and environment come from the
+// scene table (the geometry arrays are shared, with global primitive ids).
+template <bool B>
+__device__ __forceinline__ SceneLights scene_lights(const FrameParams& p, int sid) {
+    if constexpr (B) {
+        const BatchScene& b = p.batch[sid];
+        return SceneLights{p.sc, p.sc.lights + b.light_first, b.num_lights, b.env};
+    } else {
+        return SceneLights{p.sc, p.sc.lights, p.sc.num_lights, p.sc.env};
+    }
 }
 
 // The camera ray of path i of the wave (Camera::generateRay with the sample's two jitter
@@ -212,7 +212,7 @@ __global__ void k_camera(const __grid_constant__ FrameParams p, long long wave_f
 }
 
 // A wave's start when the frame's shade kernel computes its depth-0 rays itself (the kernel
-// of all materials at 128 registers, plain frames: p.cam_fused): the closest-hit and shade
+// of all materials that fetches ahead, plain frames: p.cam_fused): the closest-hit and shade
 // stages of depth 0 take each camera ray from camera_path, so no queue records are written;
 // the shade stage of depth 0 writes each path's first radiance. Without any depth, the paths'
 // radiance is zero.
@@ -346,8 +346,7 @@ __global__ void __maxnreg__(traversal_regs(W)) k_extend(const __grid_constant__ 
     float tmin = tmin0;
     RayPre r = make_raypre(V{0.f, 0.f, 0.f}, V{0.f, 0.f, 1.f});
     Hit h{FLT_MAX, 0.f, 0.f, kMissPrim};
-    SceneDevice scb;
-    if (B) scb = p.sc;
+    int root = p.sc.root;
     bool more = true;  // warp-uniform: the queue may hold rays not yet taken
     for (;;) {
         if (more) {
@@ -367,14 +366,14 @@ __global__ void __maxnreg__(traversal_regs(W)) k_extend(const __grid_constant__ 
                     int last = p.max_depth - 1;
                     if (B) {
                         const int sid = tag_scene(__float_as_int(o.w));
-                        scb = batch_scene_view(p, sid);
+                        root = p.batch[sid].root;
                         last = p.batch[sid].max_depth - 1;
                     }
                     retrace = two && depth < last;
                     second = false;
                     tmin = tmin0;
                     h = Hit{FLT_MAX, 0.f, 0.f, kMissPrim};
-                    cur = B ? scb.root : p.sc.root;
+                    cur = B ? root : p.sc.root;
                     sp = 0;
                     pend = kEmptyChild;
                     of = 0;
@@ -384,8 +383,7 @@ __global__ void __maxnreg__(traversal_regs(W)) k_extend(const __grid_constant__ 
         }
         // with no query left after a fetch, the queue is exhausted (more is false)
         if (!__any_sync(0xffffffffu, alive)) break;
-        const SceneDevice& sc = B ? scb : p.sc;
-        traverse_round<W, false, CNT>(sc.nodes, sc.prims, quant, spec, r, tmin, FLT_MAX, st, h, cur, pend, sp, alive,
+        traverse_round<W, false, CNT>(p.sc.nodes, p.sc.prims, quant, spec, r, tmin, FLT_MAX, st, h, cur, pend, sp, alive,
                                       hit_any, of, &work, Q == 2);
         // a triangle at t = tMin is inside the continuation's range, a sphere is not (triangle.cu:34
         // accepts t >= tMin, sphere.cu:16,29 need t > tMin)
@@ -398,7 +396,7 @@ __global__ void __maxnreg__(traversal_regs(W)) k_extend(const __grid_constant__ 
             second = true;
             tmin = kBounceTMin;
             h = Hit{FLT_MAX, 0.f, 0.f, kMissPrim};
-            cur = B ? scb.root : p.sc.root;
+            cur = B ? root : p.sc.root;
             sp = 0;
             pend = kEmptyChild;
             of = 0;
@@ -571,7 +569,7 @@ __device__ __forceinline__ void guide_account(const FrameParams& p, long long ti
 // emission of a Lambertian emitter with the MIS weight against the emitter sampler, else
 // nothing. Rare, so kept out of line to spare the shade stage's registers.
 // Returns the unweighted emission and its weight through `w`.
-__device__ __noinline__ V direct_hit_emission(const SceneDevice& sc, V o, V dir, float4 hd, float bsdf_pdf,
+__device__ __noinline__ V direct_hit_emission(const SceneDevice& sc, int n_choice, V o, V dir, float4 hd, float bsdf_pdf,
                                               bool nomis, bool orthonormal, float& w) {
     V point, n;
     int mat;
@@ -583,7 +581,7 @@ __device__ __noinline__ V direct_hit_emission(const SceneDevice& sc, V o, V dir,
     const Frame fr = make_frame(n);
     const V wo = normalized(to_local(fr, -dir));
     if (wo.z < 0.f) return mkv(0.f);
-    w = nomis ? 1.f : balance(bsdf_pdf, pdf_scene_light(sc, o, point, n, __float_as_int(hd.w)));
+    w = nomis ? 1.f : balance(bsdf_pdf, pdf_scene_light(sc, n_choice, o, point, n, __float_as_int(hd.w)));
     return mkv(m.emit[0], m.emit[1], m.emit[2]);
 }
 
@@ -595,25 +593,35 @@ __device__ __noinline__ V direct_hit_emission(const SceneDevice& sc, V o, V dir,
 // which measured 37% faster on the latency-bound guided shade (slit room, 1024^2).
 constexpr int kShadeGuidedBlock = 128;
 constexpr int kShadeGuidedBlocksPerSm = 8;
-// Register budget of the per-class shade kernels (k_shade_class), measured on a B200 against
-// 64, 80, 96 and 168: 64 for the Lambert, mirror, glass and miss classes (the slit room's
-// Lambert walls shaded 24% faster than in the kernel of all materials), 96 for the two
-// Beckmann classes (their sampling spills at 64; the icosphere shaded 12% faster).
-__host__ __device__ constexpr int shade_class_regs(int cls) { return cls == kMicrofacet + 1 || cls == kMetal + 1 ? 96 : 64; }
+// Register budgets of the plain shade kernels. The stage waits for memory (30% of issue slots used at
+// 128 registers, a quarter of the SM's warps), so each kernel takes the most warps its spills allow.
+// Frame ms at 1024x1024 (slit room) and 1024x1024, 64 spp (spheres):
+//   class kernels (k_shade_class)   Lambert, mirror, glass, miss 64 (56: +1.1 ms on the spheres);
+//     Beckmann classes 56 / 64 / 72 / 80 / 96: spheres 24.9 / 24.12 / 24.04 / 24.08 / 24.37, slit room
+//     73.0 / 73.1 / 73.2 / 73.3 / 73.6
+//   one kernel for all materials, fetching ahead (AHEAD)  64 / 72 / 80 / 96 / 128: spheres 24.65 / 24.49 /
+//     24.33 / 24.77 / 25.15
+//   the same without fetching ahead  56 / 64 / 72 / 80: slit room 74.2 / 74.0 / 74.4 / 75.6
+//   a scene of one material (k_shade_one)  Lambert 48 / 56 / 64 / 80 / 96: Cornell box 2.78 / 2.75 / 2.73 /
+//     2.78 / 2.91 (3.05 in the kernel for all materials); Beckmann 40 / 48 / 56 / 64 / 80: mesh at 1080p
+//     26.1 / 25.88 / 25.89 / 26.06 / 26.6 (27.2 in the kernel for all)
+constexpr bool beckmann(int type) { return type == kMicrofacet || type == kMetal; }
+constexpr int shade_class_regs(int cls) { return beckmann(cls - 1) ? 72 : 64; }
+constexpr int shade_one_regs(int type) { return beckmann(type) ? 56 : 64; }
+constexpr int kShadeAheadRegs = 80, kShadePlainRegs = 64;
 
 // CLS: -1, every slot of the queue (in material-sorted order when sorting is on); >= 0, only
 // the slots the sort put in material class CLS (0 miss, type + 1 otherwise), with that
 // class's BSDF fixed at compile time, so each class kernel holds only its own registers.
 // IPL items per lane per warp iteration: one fetch and one append atomic per warp serve
 // 32 x IPL items (the queue counters are single addresses every warp of the grid hits).
-// AHEAD (kernels with registers to spare): the warp claims its next chunk while the current
-// one shades (lane 0's atomic is read at the top of the next iteration), loads a slot's
-// random state with its other records, and issues the continuation and shadow appends'
-// atomics together, so fewer global round trips are serialised per chunk. Under a tight
-// register budget the extra live values spill and the stage slows down.
-template <bool GUIDE, bool B, int CLS, int IPL, bool AHEAD = false>
+// AHEAD: the warp claims its next chunk while the current one shades (lane 0's atomic is read at
+// the top of the next iteration) and loads a slot's random state with its other records, so
+// fewer global round trips are serialised per chunk, for a few more live registers.
+// ONLY: the material type of every surface of the scene, or -1.
+template <bool GUIDE, bool B, int CLS, int IPL, bool AHEAD = false, int ONLY = -1>
 __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long long wave_first, long long gfirst) {
-    constexpr int kType = CLS > 0 ? CLS - 1 : -1;  // the material type of a class kernel
+    constexpr int kType = CLS > 0 ? CLS - 1 : ONLY;  // the material type of a class kernel, or of the whole scene
     int count = ray_count(p, depth);
     int cls_first = 0;
     if constexpr (CLS >= 0) {  // the class's range of the sorted order
@@ -694,13 +702,12 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
             const int tag = __float_as_int(o4.w);
             const int path = tag_path(tag);
             const int sid = B ? tag_scene(tag) : 0;
-            SceneDevice scb;
-            if (B) scb = batch_scene_view(p, sid);
-            const SceneDevice& sc = B ? scb : p.sc;
+            const SceneDevice& sc = p.sc;
+            const SceneLights sl = scene_lights<B>(p, sid);
             const long long ti = GUIDE && p.guide_mode ? train_index<B>(p, sid, path, wave_first, gfirst) : -1;
             const bool last = B ? depth >= p.batch[sid].max_depth - 1 : last_frame;
             const bool guided = B ? GUIDE && p.batch[sid].guide_mode == 2 : guided_frame;
-            const bool do_nee = p.nee && sc.num_lights + (sc.env.present ? 1 : 0) > 0;
+            const bool do_nee = p.nee && sl.choices() > 0;
             const int flags = __float_as_int(b4.w);
             const V o = mkv(o4), dir = mkv(d4), beta = mkv(b4);
             const int prim = __float_as_int(h4.w);
@@ -709,7 +716,7 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
             if (split) {
                 const bool ortho = GUIDE && (B ? p.batch[sid].guide_mode : p.guide_mode);
                 float w;
-                const V Le = direct_hit_emission(sc, o, dir, q.hitd[slot], d4.w, nomis, ortho, w);
+                const V Le = direct_hit_emission(sc, sl.choices(), o, dir, q.hitd[slot], d4.w, nomis, ortho, w);
                 if (!is_zero(Le)) {
                     Ladd = beta * Le * w;
                     if (GUIDE) guide_account(p, ti, depth, lum(beta * Le), lum(Ladd), lum(Ladd));
@@ -720,9 +727,9 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
             if (miss) {
                 // escaped: environment radiance (path_tracer.cu:68-79, :162, :206, :228); a
                 // continuation that misses after a closer BSDF-direct hit adds nothing (:178-180)
-                const V Le = split ? mkv(0.f) : env_emit(sc.env, dir);
+                const V Le = split ? mkv(0.f) : env_emit(sl.env, dir);
                 if (!is_zero(Le)) {
-                    const float w = nomis ? 1.f : balance(d4.w, pdf_env_light(sc, dir));
+                    const float w = nomis ? 1.f : balance(d4.w, pdf_env_light(sl, dir));
                     Ladd = beta * Le * w;
                     if (GUIDE) guide_account(p, ti, depth, lum(beta * Le), lum(Ladd), lum(Ladd));
                 }
@@ -740,7 +747,7 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
                 // front-face emission (lambertian.cu:5-11); only Lambertian materials emit
                 if ((kType < 0 || kType == kLambertian) && !split && m.emitting && wo.z >= 0.f) {
                     const V Le = mkv(m.emit[0], m.emit[1], m.emit[2]);
-                    const float w = nomis ? 1.f : balance(d4.w, pdf_scene_light(sc, o, point, n, prim));
+                    const float w = nomis ? 1.f : balance(d4.w, pdf_scene_light(sc, sl.choices(), o, point, n, prim));
                     Ladd = beta * Le * w;
                     if (GUIDE) guide_account(p, ti, depth, lum(beta * Le), lum(Ladd), lum(Ladd));
                 }
@@ -797,7 +804,7 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
                         const float x1 = pcg_uniform(st, inc);
                         const float x2 = pcg_uniform(st, inc);
                         const float x3 = pcg_uniform(st, inc);
-                        const LightSample ls = sample_lights(sc, point, x1, x2, x3);
+                        const LightSample ls = sample_lights(sl, point, x1, x2, x3);
                         if (dot(ls.normal, ls.wi) < 0.f && ls.pdf > 0.f) {
                             const V wil = to_local(fr, ls.wi);
                             float bpdf = p.consistent_mis ? bsdf_sampling_pdf_t<kType>(m, wo, wil)
@@ -921,17 +928,24 @@ __global__ void __launch_bounds__(GUIDE ? kShadeGuidedBlock : 512, GUIDE ? kShad
 // 64 or 128 items) measured slower on every configuration: the extra live state costs more
 // warps than the contended queue counters do.
 constexpr int kShadeIpl = 1;
-// The plain shade stage over every slot of the queue (all materials) at a register budget
-// of REGS: 128 (16 warps per SM at 128-thread blocks) or 80 (24 warps, with spills), the
-// autotuner's choice per scene (the icosphere shaded 16% faster at 80, the spheres 7% slower).
-template <bool B, int REGS>
-__global__ void __maxnreg__(REGS) k_shade_all(const __grid_constant__ FrameParams p, int depth, long long wave_first,
-                                              long long gfirst) {
-    shade_body<false, B, -1, kShadeIpl, REGS >= 128>(p, depth, wave_first, gfirst);
+// The plain shade stage over every slot of the queue (all materials), fetching ahead or not: the
+// autotuner's choice per scene.
+template <bool B, bool AHEAD>
+__global__ void __maxnreg__(AHEAD ? kShadeAheadRegs : kShadePlainRegs)
+    k_shade_all(const __grid_constant__ FrameParams p, int depth, long long wave_first, long long gfirst) {
+    shade_body<false, B, -1, kShadeIpl, AHEAD>(p, depth, wave_first, gfirst);
 }
 __host__ __device__ constexpr int shade_resident(int regs, int block) {
     return 65536 / (regs * block) < 2048 / block ? (65536 / (regs * block) > 0 ? 65536 / (regs * block) : 1)
                                                  : 2048 / block;
+}
+
+// The plain shade stage over every slot of the queue in a scene whose surfaces all have material
+// type TYPE: no sorting, and the BSDF fixed at compile time.
+template <int TYPE>
+__global__ void __maxnreg__(shade_one_regs(TYPE)) k_shade_one(const __grid_constant__ FrameParams p, int depth,
+                                                              long long wave_first, long long gfirst) {
+    shade_body<false, false, -1, kShadeIpl, false, TYPE>(p, depth, wave_first, gfirst);
 }
 
 // The shade stage over one material class of a sorted queue (plain frames).
@@ -960,8 +974,6 @@ __global__ void __maxnreg__(traversal_regs(W)) k_shadow(const __grid_constant__ 
     float tmax = 0.f;
     RayPre r = make_raypre(V{0.f, 0.f, 0.f}, V{0.f, 0.f, 1.f});
     Hit h{0.f, 0.f, 0.f, kMissPrim};  // unused by any-hit queries
-    SceneDevice scb;
-    if (B) scb = p.sc;
     bool more = true;  // warp-uniform: the queue may hold rays not yet taken
     for (;;) {
         if (more) {
@@ -979,8 +991,7 @@ __global__ void __maxnreg__(traversal_regs(W)) k_shadow(const __grid_constant__ 
                     r = make_raypre(mkv(o), mkv(d));
                     tmax = o.w;
                     tag = __float_as_int(d.w);
-                    if (B) scb = batch_scene_view(p, tag_scene(tag));
-                    cur = B ? scb.root : p.sc.root;
+                    cur = B ? p.batch[tag_scene(tag)].root : p.sc.root;
                     sp = 0;
                     pend = kEmptyChild;
                     of = 0;
@@ -990,8 +1001,7 @@ __global__ void __maxnreg__(traversal_regs(W)) k_shadow(const __grid_constant__ 
             }
         }
         if (!__any_sync(0xffffffffu, alive)) break;
-        const SceneDevice& sc = B ? scb : p.sc;
-        traverse_round<W, true, CNT>(sc.nodes, sc.prims, quant, spec, r, kShadowTMin, tmax, st, h, cur, pend, sp, alive,
+        traverse_round<W, true, CNT>(p.sc.nodes, p.sc.prims, quant, spec, r, kShadowTMin, tmax, st, h, cur, pend, sp, alive,
                                      occ, of, &work, Q == 2, near);
         if (slot >= 0 && !alive) {  // the query ended: occluded, or the stack ran empty
             const int i = slot;
@@ -1340,14 +1350,36 @@ cudaError_t resident_grid(const void* kernel, int block, size_t smem, const Fram
     return e;
 }
 
+using ShadeKernel = void (*)(FrameParams, int, long long, long long);
+// The material type of a scene with exactly one (class mask bit type + 1; bit 0, misses, aside), else -1.
+int one_material(int class_mask) {
+    const int m = class_mask >> 1;
+    if (m == 0 || (m & (m - 1))) return -1;
+    int t = 0;
+    while (!(m & (1 << t))) t++;
+    return t;
+}
+ShadeKernel one_kernel(int type) {
+    switch (type) {
+        case kLambertian: return k_shade_one<kLambertian>;
+        case kMirror: return k_shade_one<kMirror>;
+        case kGlass: return k_shade_one<kGlass>;
+        case kMicrofacet: return k_shade_one<kMicrofacet>;
+        default: return k_shade_one<kMetal>;
+    }
+}
+
 template <int W, bool CNT, bool B>
 cudaError_t enqueue_waves(const FrameParams& p_in, const WaveRange* waves, int nwaves, cudaStream_t stream,
                           StageMarks* marks, const SideStream* side) {
     // depth-0 rays are computed where they are used when every depth-0 stage can do so: plain
-    // frames whose shade stage is the kernel of all materials at 128 registers
+    // frames whose shade stage is the kernel of all materials that fetches ahead
     FrameParams p = p_in;
     const bool classes = p.shape.shade_kernel == kShadeClasses && p.shape.sort_materials && p.class_mask;
-    p.cam_fused = p.shape.fuse_camera && !p.guide_mode && !classes && p.shape.shade_kernel != kShadeAll80 ? 1 : 0;
+    // a scene of one material has its own kernel, unless the class kernels run
+    const int one = !B && !p.guide_mode && !classes ? one_material(p.class_mask) : -1;
+    p.cam_fused =
+        p.shape.fuse_camera && !p.guide_mode && !classes && one < 0 && p.shape.shade_kernel != kShadeAllPlain ? 1 : 0;
     // shadow stage of depth d on the side stream: forked after the shade stage of d, joined
     // before the shade stage of d + 1 (which adds to the same path radiance after it); the
     // closest-hit stage of d + 1 runs beside it
@@ -1409,15 +1441,18 @@ cudaError_t enqueue_waves(const FrameParams& p_in, const WaveRange* waves, int n
             if (p.guide_mode)
                 k_shade<true, B><<<p.num_sms * kShadeGuidedBlocksPerSm, kShadeGuidedBlock, 0, stream>>>(
                     p, d, wave_first, w.guided_first);
-            else if (p.shape.shade_kernel == kShadeClasses && p.shape.sort_materials && p.class_mask)
+            else if (classes)
                 e = enqueue_class_shades<B>(p, d, wave_first, w.guided_first, stream,
                                             concurrent && !marks && side->cls ? side : nullptr);
-            else if (p.shape.shade_kernel == kShadeAll80)
-                k_shade_all<B, 80><<<p.num_sms * shade_resident(80, p.shape.block_shade), p.shape.block_shade, 0,
-                                     stream>>>(p, d, wave_first, w.guided_first);
-            else
-                k_shade_all<B, 128><<<p.num_sms * shade_resident(128, p.shape.block_shade), p.shape.block_shade, 0,
-                                      stream>>>(p, d, wave_first, w.guided_first);
+            else {
+                const int regs = one >= 0 ? shade_one_regs(one)
+                                 : p.shape.shade_kernel == kShadeAllPlain ? kShadePlainRegs : kShadeAheadRegs;
+                const ShadeKernel shade = one >= 0 ? one_kernel(one)
+                                          : p.shape.shade_kernel == kShadeAllPlain ? k_shade_all<B, false>
+                                                                                   : k_shade_all<B, true>;
+                shade<<<p.num_sms * shade_resident(regs, p.shape.block_shade), p.shape.block_shade, 0, stream>>>(
+                    p, d, wave_first, w.guided_first);
+            }
             if (e != cudaSuccess) return e;
             mark(kStageShade);
             if (p.nee && d < p.max_depth - 1) {

@@ -99,7 +99,7 @@ struct LaunchShape {
     int sort_rays = 0;        // continuation rays extended in (origin cell, direction octant) order
     int refill_idle = 16;     // traversal stages: a warp fetches new rays once this many lanes are idle
     int speculate = 0;        // kSpeculate* bits: stages that park a lane's first leaf and descend on
-    int shade_kernel = 1;     // plain frames' shade stage: kShadeAll128, kShadeClasses, kShadeAll80
+    int shade_kernel = 1;     // plain frames' shade stage: kShadeAllAhead, kShadeClasses, kShadeAllPlain
     int overlap_shadow = 1;   // shadow stage of depth d on the side stream beside extend of d + 1
     int shadow_near = 0;      // shadow stage: a node's hit children visited nearest first (else in order)
     int fuse_camera = 1;      // depth-0 rays computed where used when the shade kernel allows (cam_fused)
@@ -118,9 +118,9 @@ struct SideStream {
     cudaEvent_t* cls_done = nullptr;  // recorded on each class stream after its kernel
 };
 
-constexpr int kShadeAll128 = 0;  // one kernel for all materials, 128 registers
+constexpr int kShadeAllAhead = 0;  // one kernel for all materials, fetching its queue ahead
 constexpr int kShadeClasses = 1; // material-sorted frames: one kernel per material class present
-constexpr int kShadeAll80 = 2;   // one kernel for all materials, 80 registers
+constexpr int kShadeAllPlain = 2;  // one kernel for all materials, more warps resident
 
 constexpr int kSpeculateExtend = 1;  // closest-hit stage
 constexpr int kSpeculateShadow = 2;  // shadow (any-hit) stage

@@ -124,17 +124,18 @@ typedef struct pt_launch_config {
                               stage only, 4 shadow stage only */
     int split_shade;       /* the shade stage of frames without guiding: 1 one kernel per material
                               class present, each compiled for its BSDF only (material-sorted
-                              frames; default), 2 one kernel for all materials at 128 registers,
-                              3 the same at 80 registers (more resident warps, some spills);
-                              images are the same either way */
+                              frames; default), 2 one kernel for all materials that fetches its
+                              queue ahead, 3 the same without fetching ahead (more resident
+                              warps); without the class kernels, a scene of one material runs a
+                              kernel compiled for it; images are the same either way */
     int overlap_shadow;    /* 1: the shadow stage of depth d runs on a second stream beside the
                               closest-hit stage of depth d + 1, each filling the other's tail
                               (default; the shade stage of depth d + 1 waits for both), 2: one
                               stream; images are the same either way */
     int shadow_order;      /* shadow stage: 1 a node's hit children are visited nearest first, 2 in
                               the node's order (default); the same occlusion results either way */
-    int fuse_camera;       /* 1 (default): in plain frames whose shade stage is the one kernel at 128
-                              registers, the closest-hit and shade stages of depth 0 compute each
+    int fuse_camera;       /* 1 (default): in plain frames whose shade stage is the one kernel that
+                              fetches ahead, the closest-hit and shade stages of depth 0 compute each
                               camera ray from its path index instead of reading it from a queue
                               that a camera stage wrote; 2: always queued; the same images */
 } pt_launch_config;
@@ -152,8 +153,8 @@ typedef struct pt_tune_result {
     int from_cache;
     int sort_rays;          /* 1 on, 2 off */
     int speculate;          /* as pt_launch_config.speculate: 1 both stages, 2 off, 3 closest hit, 4 shadow */
-    int split_shade;        /* as pt_launch_config.split_shade: 1 per-class kernels, 2 one kernel (128
-                               registers), 3 one kernel (80 registers) */
+    int split_shade;        /* as pt_launch_config.split_shade: 1 per-class kernels, 2 one kernel
+                               (fetching ahead), 3 one kernel (not) */
     int max_leaf;           /* primitives per BVH leaf (2, 4, 8 or 16; as pt_set_bvh) */
     int bvh_builder;        /* as pt_set_bvh_builder: 0 host binned SAH, 2 GPU PLOC (single scenes) */
     int shadow_order;       /* as pt_launch_config.shadow_order: 1 nearest first, 2 the node's order */
