@@ -213,9 +213,16 @@ __device__ __forceinline__ float cdf_pmf(const float* cdf, int i) {
     return i == 0 ? c : c - __ldg(cdf + i - 1);
 }
 // Distribution::sample (distribution.h:197-224): first index with xi < cdf[i]; for xi == 1
-// the first index whose cdf equals 1. Binary search over the monotone CDF.
-__device__ __forceinline__ int cdf_sample(const float* cdf, int n, float xi) {
+// the first index whose cdf equals 1. Binary search over the monotone CDF, between the variate's
+// cut points when there are any (the same index: the answer is monotone in xi, and xi * kCdfCuts
+// is exact).
+__device__ __forceinline__ int cdf_sample(const float* cdf, const uint16_t* cut, int n, float xi) {
     int lo = 0, hi = n;
+    if (cut) {
+        const int k = min((int)(xi * kCdfCuts), kCdfCuts - 1);
+        lo = __ldg(cut + k);
+        hi = __ldg(cut + k + 1);
+    }
     while (lo < hi) {
         const int mid = (lo + hi) >> 1;
         if (xi < __ldg(cdf + mid)) hi = mid; else lo = mid + 1;
@@ -249,8 +256,9 @@ __device__ __forceinline__ float env_pdf_dir(const EnvDevice& e, V w) {
 // uniform point inside the texel when `continuous` is set.
 __device__ __forceinline__ V env_sample_dir(const EnvDevice& e, float xi1, float xi2, float& pdf, float cx = 0.5f,
                                             float cy = 0.5f) {
-    const int y = cdf_sample(e.marg_cdf, e.height, xi1);
-    const int x = cdf_sample(e.cond_cdf + (size_t)y * e.width, e.width, xi2);
+    const int y = cdf_sample(e.marg_cdf, e.marg_cut, e.height, xi1);
+    const uint16_t* row_cut = e.cond_cut ? e.cond_cut + (size_t)y * (kCdfCuts + 1) : nullptr;
+    const int x = cdf_sample(e.cond_cdf + (size_t)y * e.width, row_cut, e.width, xi2);
     const float phi = ((x + cx) / e.width) * kPiF * 2.f;
     const float theta = ((y + cy) / e.height) * kPiF;
     float sp, cp, st, ct;

@@ -752,6 +752,18 @@ int Session::upload_materials() {
     return PT_OK;
 }
 
+// Cut points of an environment's marginal CDF, then of its rows' (none for maps too large for
+// their 16-bit indices).
+int Session::build_env_cuts(DevBuf& cuts, const DevBuf& marg, const DevBuf& cond, int w, int h) {
+    if (!env_cuts_fit(w, h)) return PT_OK;
+    int r;
+    if ((r = check_cuda(cuts.alloc((size_t)(h + 1) * (kCdfCuts + 1) * sizeof(uint16_t)), "environment cut points")))
+        return r;
+    uint16_t* c = cuts.as<uint16_t>();
+    if ((r = check_cuda(build_cdf_cuts(marg.as<float>(), h, 1, c, stream_), "environment cut points"))) return r;
+    return check_cuda(build_cdf_cuts(cond.as<float>(), w, h, c + kCdfCuts + 1, stream_), "environment cut points");
+}
+
 int Session::upload_scene() {
     int r;
     const int nt = scene_.num_tri();
@@ -777,6 +789,7 @@ int Session::upload_scene() {
         if ((r = check_cuda(upload(d_env_marg_, env_cdf_.marg, stream_), "upload environment CDF"))) return r;
         if ((r = check_cuda(upload(d_env_cond_, env_cdf_.cond, stream_), "upload environment CDF"))) return r;
         if ((r = check_cuda(upload(d_env_row_, env_cdf_.row_mass, stream_), "upload environment CDF"))) return r;
+        if ((r = build_env_cuts(d_env_cut_, d_env_marg_, d_env_cond_, scene_.env_w, scene_.env_h))) return r;
     }
     if (gpu_tree) {  // the wide BVH built on the device from the uploaded primitives
         cudaEvent_t e0, e1;
@@ -878,6 +891,7 @@ SceneDevice Session::scene_view() const {
         v.env.marg_cdf = d_env_marg_.as<float>();
         v.env.cond_cdf = d_env_cond_.as<float>();
         v.env.row_mass = d_env_row_.as<float>();
+        set_env_cuts(v.env, d_env_cut_, scene_.env_w, scene_.env_h);
         v.env.width = scene_.env_w;
         v.env.height = scene_.env_h;
         v.env.total_mass = env_cdf_.total;

@@ -45,6 +45,12 @@ cudaError_t upload(DevBuf& b, const std::vector<T>& v, cudaStream_t st) {
     return cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st);
 }
 
+inline bool env_cuts_fit(int w, int h) { return w <= kCdfCutMax && h <= kCdfCutMax; }
+inline void set_env_cuts(EnvDevice& e, const DevBuf& cuts, int w, int h) {
+    e.marg_cut = env_cuts_fit(w, h) ? cuts.as<uint16_t>() : nullptr;
+    e.cond_cut = e.marg_cut ? e.marg_cut + kCdfCuts + 1 : nullptr;
+}
+
 class Session {
 public:
     Session(int w, int h);
@@ -156,7 +162,8 @@ private:
     DevBuf d_qnodes_, d_qfail_;
     int bvh_quant_ = 0;
     DevBuf d_nodes_, d_prims_, d_tri_p_, d_tri_n_, d_tri_mat_, d_sph_, d_sph_mat_, d_mats_, d_lights_;
-    DevBuf d_env_rgba_, d_env_marg_, d_env_cond_, d_env_row_;
+    DevBuf d_env_rgba_, d_env_marg_, d_env_cond_, d_env_row_, d_env_cut_;
+    int build_env_cuts(DevBuf& cuts, const DevBuf& marg, const DevBuf& cond, int w, int h);
     // frame state
     DevBuf d_pass_, d_accum_, d_rgba8_;
     DevBuf d_q_[2][6];
@@ -239,7 +246,7 @@ private:
     std::vector<BatchHost> batch_;
     std::vector<BatchSpec> batch_specs_;
     std::vector<WaveRange> batch_waves_;
-    std::vector<std::unique_ptr<DevBuf[]>> d_batch_env_;  // per scene: rgba, marg, cond, row
+    std::vector<std::unique_ptr<DevBuf[]>> d_batch_env_;  // per scene: rgba, marg, cond, row, cuts
     DevBuf d_batch_, d_batch_path_base_, d_batch_pixel_base_;
     BatchScene* h_batch_ = nullptr;  // pinned
     int batch_max_depth_ = 0;

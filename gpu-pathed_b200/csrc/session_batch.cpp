@@ -144,7 +144,7 @@ int Session::upload_batch() {
     const int n = (int)batch_.size();
     d_batch_env_.clear();
     for (int i = 0; i < n; i++) {
-        d_batch_env_.emplace_back(new DevBuf[4]);
+        d_batch_env_.emplace_back(new DevBuf[5]);
         const BatchHost& h = batch_[i];
         if (h.env_w > 0) {
             DevBuf* e = d_batch_env_.back().get();
@@ -152,6 +152,7 @@ int Session::upload_batch() {
             if ((r = check_cuda(upload(e[1], h.env_cdf.marg, stream_), "upload environment CDF"))) return r;
             if ((r = check_cuda(upload(e[2], h.env_cdf.cond, stream_), "upload environment CDF"))) return r;
             if ((r = check_cuda(upload(e[3], h.env_cdf.row_mass, stream_), "upload environment CDF"))) return r;
+            if ((r = build_env_cuts(e[4], e[1], e[2], h.env_w, h.env_h))) return r;
         }
     }
     if (!h_batch_ && (r = check_cuda(cudaMallocHost((void**)&h_batch_, kMaxBatchScenes * sizeof(BatchScene)),
@@ -179,6 +180,7 @@ int Session::upload_batch() {
             b.env.marg_cdf = e[1].as<float>();
             b.env.cond_cdf = e[2].as<float>();
             b.env.row_mass = e[3].as<float>();
+            set_env_cuts(b.env, e[4], h.env_w, h.env_h);
             b.env.width = h.env_w;
             b.env.height = h.env_h;
             b.env.total_mass = h.env_cdf.total;

@@ -1696,6 +1696,21 @@ __global__ void __launch_bounds__(kQueryBlock)
     }
 }
 
+// One block per CDF; thread k finds cut k.
+__global__ void k_cdf_cuts(const float* __restrict__ cdf, int n, uint16_t* __restrict__ cuts) {
+    const int k = threadIdx.x;
+    if (k > kCdfCuts) return;
+    const float* row = cdf + (size_t)blockIdx.x * n;
+    const float xi = (float)k / kCdfCuts;
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (xi < row[mid]) hi = mid;
+        else lo = mid + 1;
+    }
+    cuts[(size_t)blockIdx.x * (kCdfCuts + 1) + k] = (uint16_t)lo;
+}
+
 template <int W>
 __global__ void k_hit_test(SceneDevice sc, CameraParams cam, StackShape shape, int x, int y, int* out, int* overflow) {
     extern __shared__ int2 stk[];
@@ -1748,6 +1763,12 @@ cudaError_t enqueue_batch_frame(const FrameParams& p, const WaveRange* waves, in
                            : enqueue_waves<8, false, true>(p, waves, nwaves, stream, marks, side);
         default: return cudaErrorInvalidValue;
     }
+}
+
+cudaError_t build_cdf_cuts(const float* cdf, int n, int rows, uint16_t* cuts, cudaStream_t stream) {
+    if (n < 1 || n > kCdfCutMax || rows < 1) return cudaErrorInvalidValue;
+    k_cdf_cuts<<<rows, 288, 0, stream>>>(cdf, n, cuts);
+    return cudaGetLastError();
 }
 
 cudaError_t configure_guide_infer() {

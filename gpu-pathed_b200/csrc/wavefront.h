@@ -252,6 +252,9 @@ cudaError_t enqueue_batch_frame(const FrameParams& p, const WaveRange* waves, in
 cudaError_t enqueue_frame(const FrameParams& p, cudaStream_t stream, StageMarks* marks = nullptr,
                           const SideStream* side = nullptr);
 
+// Cut points (kCdfCuts + 1 per row) of `rows` CDFs of n <= kCdfCutMax values each.
+cudaError_t build_cdf_cuts(const float* cdf, int n, int rows, uint16_t* cuts, cudaStream_t stream);
+
 // Raise the dynamic shared-memory limit of the traversal kernels to `bytes`.
 cudaError_t configure_traversal_smem(size_t bytes);
 // Opt the guide inference kernel into its dynamic shared memory (weights + 8 warps x 32 rows).
