@@ -47,7 +47,7 @@ __host__ __device__ __forceinline__ float unord_float(unsigned u) {
 }
 
 struct PrimIn {
-    const float4* tri_p;  // 3 per triangle
+    const float4* tri;  // kTriF4 per triangle, the vertices first
     const float4* sph;    // centre, radius
     int nt, ns;
 };
@@ -64,7 +64,7 @@ __global__ void k_lb_boxes(PrimIn in, float4* box_lo, float4* box_hi, float4* ce
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float bl[3], bh[3], c[3];
         if (i < in.nt) {
-            const float4 a = in.tri_p[3 * i], b = in.tri_p[3 * i + 1], d = in.tri_p[3 * i + 2];
+            const float4 a = in.tri[kTriF4 * i], b = in.tri[kTriF4 * i + 1], d = in.tri[kTriF4 * i + 2];
             bl[0] = fminf(fminf(a.x, b.x), d.x); bh[0] = fmaxf(fmaxf(a.x, b.x), d.x);
             bl[1] = fminf(fminf(a.y, b.y), d.y); bh[1] = fmaxf(fmaxf(a.y, b.y), d.y);
             bl[2] = fminf(fminf(a.z, b.z), d.z); bh[2] = fmaxf(fmaxf(a.z, b.z), d.z);
@@ -306,7 +306,7 @@ __global__ void k_lb_prims(const int* ids, int n, PrimIn in, float4* prims) {
     const int p = ids[e];
     float4 r0, r1, r2;
     if (p < in.nt) {
-        const float4 v0 = in.tri_p[3 * p], v1 = in.tri_p[3 * p + 1], v2 = in.tri_p[3 * p + 2];
+        const float4 v0 = in.tri[kTriF4 * p], v1 = in.tri[kTriF4 * p + 1], v2 = in.tri[kTriF4 * p + 2];
         r0 = make_float4(v0.x, v0.y, v0.z, __int_as_float(p));
         // e1, e2: the single-precision subtractions Triangle::hit performs
         r1 = make_float4(__fsub_rn(v1.x, v0.x), __fsub_rn(v1.y, v0.y), __fsub_rn(v1.z, v0.z), 0.f);
@@ -485,7 +485,7 @@ __global__ void k_ploc_order(int n, const int* sids, const int* first, int* dfs_
 
 }  // namespace
 
-cudaError_t gpu_build_bvh(const float4* tri_p, int nt, const float4* sph, int ns, int width, int max_leaf,
+cudaError_t gpu_build_bvh(const float4* tri, int nt, const float4* sph, int ns, int width, int max_leaf,
                           GpuBvhScratch& sc, DevBuf& nodes_out, DevBuf& prims_out, GpuBvhInfo& info,
                           cudaStream_t st, int algorithm) {
     const int n = nt + ns;
@@ -503,7 +503,7 @@ cudaError_t gpu_build_bvh(const float4* tri_p, int nt, const float4* sph, int ns
     const size_t node_bytes = width == 2 ? sizeof(BvhNode<2>) : width == 4 ? sizeof(BvhNode<4>) : sizeof(BvhNode<8>);
     if ((e = nodes_out.alloc((size_t)n * node_bytes)) || (e = prims_out.alloc((size_t)n * 3 * sizeof(float4))))
         return e;
-    const PrimIn in{tri_p, sph, nt, ns};
+    const PrimIn in{tri, sph, nt, ns};
     unsigned* bounds = sc.bounds.as<unsigned>();
     k_lb_bounds_init<<<1, 32, 0, st>>>(bounds);
     k_lb_boxes<<<256, 256, 0, st>>>(in, sc.box_lo.as<float4>(), sc.box_hi.as<float4>(), sc.cen.as<float4>(), bounds);
@@ -706,20 +706,20 @@ __global__ void k_quantize_nodes(const BvhNode<W>* __restrict__ in, int n, uint3
 }  // namespace
 
 // Triangle leaf entries for the watertight test: (p0, id) (p1) (p2), the original vertices
-// (tri_p, 3 float4 per triangle) in place of the edges e1, e2; sphere entries are unchanged.
+// (the first three float4 of `tri`'s records) in place of the edges e1, e2; sphere entries are unchanged.
 // Shared vertices keep their exact values, which the test's watertightness relies on.
-__global__ void k_prims_vertices(float4* __restrict__ prims, int n, const float4* __restrict__ tri_p) {
+__global__ void k_prims_vertices(float4* __restrict__ prims, int n, const float4* __restrict__ tri) {
     const int e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= n) return;
     const int id = __float_as_int(prims[3 * e].w);
     if (id < 0) return;
-    prims[3 * e + 1] = tri_p[3 * (size_t)id + 1];
-    prims[3 * e + 2] = tri_p[3 * (size_t)id + 2];
+    prims[3 * e + 1] = tri[kTriF4 * (size_t)id + 1];
+    prims[3 * e + 2] = tri[kTriF4 * (size_t)id + 2];
 }
 
-cudaError_t prims_to_vertices(float4* prims, int n, const float4* tri_p, cudaStream_t st) {
+cudaError_t prims_to_vertices(float4* prims, int n, const float4* tri, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    k_prims_vertices<<<(n + 255) / 256, 256, 0, st>>>(prims, n, tri_p);
+    k_prims_vertices<<<(n + 255) / 256, 256, 0, st>>>(prims, n, tri);
     return cudaGetLastError();
 }
 

@@ -28,12 +28,12 @@ struct GpuBvhInfo {
 // nodes_out, leaf entries (3 float4 each; Morton order for the LBVH, the tree's depth-first
 // order for PLOC) into prims_out. Synchronises `st` once per tree level of the collapse and,
 // for PLOC, once per clustering pass.
-cudaError_t gpu_build_bvh(const float4* tri_p, int nt, const float4* sph, int ns, int width, int max_leaf,
+cudaError_t gpu_build_bvh(const float4* tri, int nt, const float4* sph, int ns, int width, int max_leaf,
                           GpuBvhScratch& scratch, DevBuf& nodes_out, DevBuf& prims_out, GpuBvhInfo& info,
                           cudaStream_t st, int algorithm = kGpuBvhLbvh);
 
 // Rewrite the n leaf entries' triangles as (p0, id) (p1) (p2) for the watertight test.
-cudaError_t prims_to_vertices(float4* prims, int n, const float4* tri_p, cudaStream_t st);
+cudaError_t prims_to_vertices(float4* prims, int n, const float4* tri, cudaStream_t st);
 
 // Quantized copy (qnode_bytes(width) per node, width 4 or 8) of `num_nodes` BvhNode<width>
 // nodes on the device. `fail` (device int) is set when a node cannot be quantized

@@ -304,9 +304,10 @@ __device__ __forceinline__ LightSample sample_lights(const SceneLights& sl, V p,
         float area_pdf;
         int mat;
         if (lr.type == kTriangle) {
-            const V p0 = mkv(__ldg(sc.tri_p + 3 * lr.index + 0));
-            const V p1 = mkv(__ldg(sc.tri_p + 3 * lr.index + 1));
-            const V p2 = mkv(__ldg(sc.tri_p + 3 * lr.index + 2));
+            const float4 p0m = __ldg(sc.tri + kTriF4 * lr.index + 0);
+            const V p0 = mkv(p0m);
+            const V p1 = mkv(__ldg(sc.tri + kTriF4 * lr.index + 1));
+            const V p2 = mkv(__ldg(sc.tri + kTriF4 * lr.index + 2));
             const float sr = sqrtf(xi2);
             const float a = 1.f - sr;
             const float b = sr * (1.f - xi3);
@@ -314,7 +315,7 @@ __device__ __forceinline__ LightSample sample_lights(const SceneLights& sl, V p,
             point = p0 * a + p1 * b + p2 * c;
             normal = normalized(cross(p1 - p0, p2 - p0));
             area_pdf = 1.f / tri_area(p0, p1, p2);
-            mat = __ldg(sc.tri_mat + lr.index);
+            mat = __float_as_int(p0m.w);
         } else {
             const float4 s = __ldg(sc.sph + lr.index);
             const float z = xi2 * 2.f - 1.f;
@@ -358,9 +359,9 @@ __device__ __forceinline__ float pdf_scene_light(const SceneDevice& sc, int n_ch
                                                  int prim) {
     float area_pdf;
     if (prim >= 0) {
-        const V p0 = mkv(__ldg(sc.tri_p + 3 * prim + 0));
-        const V p1 = mkv(__ldg(sc.tri_p + 3 * prim + 1));
-        const V p2 = mkv(__ldg(sc.tri_p + 3 * prim + 2));
+        const V p0 = mkv(__ldg(sc.tri + kTriF4 * prim + 0));
+        const V p1 = mkv(__ldg(sc.tri + kTriF4 * prim + 1));
+        const V p2 = mkv(__ldg(sc.tri + kTriF4 * prim + 2));
         area_pdf = 1.f / tri_area(p0, p1, p2);
     } else {
         const float4 s = __ldg(sc.sph + ~prim);

@@ -21,6 +21,27 @@
 
 namespace pt {
 
+// 32-byte loads and stores (one instruction and one full sector per lane on sm_100a; 32-byte
+// aligned). The load names 64-bit elements: with v8.f32 ptxas 12.9 crashes on the shade kernels.
+struct F8 {
+    float4 a, b;
+};
+__device__ __forceinline__ F8 load8(const float4* p) {
+    F8 v;
+    double d0, d1, d2, d3;
+    asm("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(d0), "=d"(d1), "=d"(d2), "=d"(d3) : "l"(p));
+    v.a = make_float4(__int_as_float(__double2loint(d0)), __int_as_float(__double2hiint(d0)),
+                      __int_as_float(__double2loint(d1)), __int_as_float(__double2hiint(d1)));
+    v.b = make_float4(__int_as_float(__double2loint(d2)), __int_as_float(__double2hiint(d2)),
+                      __int_as_float(__double2loint(d3)), __int_as_float(__double2hiint(d3)));
+    return v;
+}
+__device__ __forceinline__ void store8(float4* p, float4 a, float4 b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
+
 constexpr int kMissPrim = 0x7fffffff;  // no hit
 // Relative slack applied to box-interval ends: boxes are visited when they might contain a
 // hit the primitive test would accept (never culls what the linear scan reports).

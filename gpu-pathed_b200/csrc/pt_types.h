@@ -5,7 +5,7 @@
 //   * BVH primitive refs  : 3 x float4 per leaf entry, in leaf order
 //       triangle: (p0.xyz, id)  (e1.xyz, 0)  (e2.xyz, 0)      id >= 0 is the triangle index
 //       sphere  : (c.xyz, ~id)  (r, 0, 0, 0) (0, 0, 0, 0)     ~id < 0 encodes the sphere index
-//   * triangle shading data in original (reference) order: p0,p1,p2 and n0,n1,n2 as float4
+//   * triangle shading data in original (reference) order: (p0, material) p1 p2 n0 n1 n2 as float4
 //   * materials, emitter list, equirect environment (RGBA FP32) + its marginal/conditional CDF
 //
 // The triangle/sphere records keep the reference's per-primitive semantics
@@ -132,15 +132,16 @@ struct LightRef {
     int index;
 };
 
+constexpr int kTriF4 = 6;  // three aligned 32-byte sectors per triangle, read with three 256-bit loads
+
 // Everything a kernel needs to see of a loaded scene (passed by value as a kernel argument).
 struct SceneDevice {
     const float4* nodes;       // BvhNode<W> array viewed as float4
     const float4* prims;       // 3 float4 per leaf entry
-    const float4* tri_p;       // 3 float4 per triangle: p0, p1, p2 (original order)
-    const float4* tri_n;       // 3 float4 per triangle: n0, n1, n2
-    const int* tri_mat;        // per triangle material id
+    const float4* tri;         // kTriF4 float4 per triangle (original order): (p0, material id) p1 p2 n0 n1 n2
     const float4* sph;         // per sphere: center.xyz, radius
     const int* sph_mat;        // per sphere material id
+    const uint8_t* prim_class; // material class (type + 1) of every triangle, then of every sphere
     const Material* mats;
     const LightRef* lights;
     EnvDevice env;

@@ -747,6 +747,8 @@ int Session::upload_materials() {
     int r;
     if ((r = check_cuda(upload(d_mats_, scene_.mats, stream_), "upload materials"))) return r;
     if ((r = check_cuda(upload(d_lights_, lights_, stream_), "upload lights"))) return r;
+    if ((r = check_cuda(d_class_.alloc((size_t)scene_.num_tri() + scene_.num_sph()), "material classes"))) return r;
+    if ((r = check_cuda(build_prim_classes(scene_view(), d_class_.as<uint8_t>(), stream_), "material classes"))) return r;
     if ((r = check_cuda(cudaStreamSynchronize(stream_), "upload materials"))) return r;
     mats_dirty_ = false;
     return PT_OK;
@@ -767,21 +769,30 @@ int Session::build_env_cuts(DevBuf& cuts, const DevBuf& marg, const DevBuf& cond
 int Session::upload_scene() {
     int r;
     const int nt = scene_.num_tri();
-    std::vector<float> tp((size_t)nt * 12, 0.f), tn((size_t)nt * 12, 0.f);
-    for (int i = 0; i < nt; i++)
-        for (int v = 0; v < 3; v++)
-            for (int k = 0; k < 3; k++) {
-                tp[(size_t)i * 12 + v * 4 + k] = scene_.tri_p[(size_t)i * 9 + v * 3 + k];
-                tn[(size_t)i * 12 + v * 4 + k] = scene_.tri_n[(size_t)i * 9 + v * 3 + k];
-            }
     const bool gpu_tree = bvh_gpu_ != 0 && !batch_mode();
     if (!gpu_tree) {
         if ((r = check_cuda(upload(d_nodes_, bvh_.nodes, stream_), "upload BVH nodes"))) return r;
         if ((r = check_cuda(upload(d_prims_, bvh_.prims, stream_), "upload BVH primitives"))) return r;
     }
-    if ((r = check_cuda(upload(d_tri_p_, tp, stream_), "upload triangles"))) return r;
-    if ((r = check_cuda(upload(d_tri_n_, tn, stream_), "upload normals"))) return r;
-    if ((r = check_cuda(upload(d_tri_mat_, scene_.tri_mat, stream_), "upload triangle materials"))) return r;
+    if ((r = check_cuda(d_tri_.alloc((size_t)nt * kTriF4 * sizeof(float4)), "triangles"))) return r;
+    if (nt > 0) {  // the scene's own arrays, packed into records on the device
+        const size_t floats = (size_t)nt * 9;
+        if ((r = check_cuda(d_scratch_.alloc((2 * floats + nt) * 4), "scratch"))) return r;
+        float* p = d_scratch_.as<float>();
+        if ((r = check_cuda(cudaMemcpyAsync(p, scene_.tri_p.data(), floats * 4, cudaMemcpyHostToDevice, stream_),
+                            "upload triangles")))
+            return r;
+        if ((r = check_cuda(cudaMemcpyAsync(p + floats, scene_.tri_n.data(), floats * 4, cudaMemcpyHostToDevice,
+                                            stream_),
+                            "upload normals")))
+            return r;
+        int* mat = reinterpret_cast<int*>(p + 2 * floats);
+        if ((r = check_cuda(cudaMemcpyAsync(mat, scene_.tri_mat.data(), (size_t)nt * 4, cudaMemcpyHostToDevice, stream_),
+                            "upload triangle materials")))
+            return r;
+        if ((r = check_cuda(pack_triangles(p, p + floats, mat, nt, d_tri_.as<float4>(), stream_), "pack triangles")))
+            return r;
+    }
     if ((r = check_cuda(upload(d_sph_, scene_.sph, stream_), "upload spheres"))) return r;
     if ((r = check_cuda(upload(d_sph_mat_, scene_.sph_mat, stream_), "upload sphere materials"))) return r;
     if (scene_.env_w > 0) {
@@ -797,7 +808,7 @@ int Session::upload_scene() {
         if ((r = check_cuda(cudaEventCreate(&e1), "cudaEventCreate"))) return r;
         cudaEventRecord(e0, stream_);
         GpuBvhInfo info;
-        const cudaError_t be = gpu_build_bvh(d_tri_p_.as<float4>(), nt, d_sph_.as<float4>(), scene_.num_sph(),
+        const cudaError_t be = gpu_build_bvh(d_tri_.as<float4>(), nt, d_sph_.as<float4>(), scene_.num_sph(),
                                              bvh_width_, bvh_leaf_, gbvh_, d_nodes_, d_prims_, info, stream_, bvh_gpu_);
         cudaEventRecord(e1, stream_);
         cudaEventSynchronize(e1);
@@ -816,7 +827,7 @@ int Session::upload_scene() {
     }
     if (watertight_) {  // triangle entries carry their vertices for the watertight test
         const int entries = gpu_tree ? nt + scene_.num_sph() : (int)(bvh_.prims.size() / 12);
-        if ((r = check_cuda(prims_to_vertices(d_prims_.as<float4>(), entries, d_tri_p_.as<float4>(), stream_),
+        if ((r = check_cuda(prims_to_vertices(d_prims_.as<float4>(), entries, d_tri_.as<float4>(), stream_),
                             "watertight leaf entries")))
             return r;
     }
@@ -872,9 +883,8 @@ SceneDevice Session::scene_view() const {
     v.nodes = qn ? d_qnodes_.as<float4>() : d_nodes_.as<float4>();
     v.node_q = qn;
     v.prims = d_prims_.as<float4>();
-    v.tri_p = d_tri_p_.as<float4>();
-    v.tri_n = d_tri_n_.as<float4>();
-    v.tri_mat = d_tri_mat_.as<int>();
+    v.tri = d_tri_.as<float4>();
+    v.prim_class = d_class_.as<uint8_t>();
     v.sph = d_sph_.as<float4>();
     v.sph_mat = d_sph_mat_.as<int>();
     v.mats = d_mats_.as<Material>();
@@ -947,13 +957,13 @@ int Session::ensure_frame_buffers(int spp) {
     }
     const size_t f4 = cap * sizeof(float4);
     for (int k = 0; k < 2; k++) {
-        for (int a = 0; a < 6; a++) {
-            const size_t bytes = a == 3 ? cap * sizeof(uint2) : a == 5 ? cap * sizeof(int) : f4;
+        for (int a = 0; a < 4; a++) {
+            const size_t bytes = a < 2 ? 2 * f4 : a == 2 ? f4 : cap * sizeof(int);
             if ((r = check_cuda(d_q_[k][a].alloc(bytes), "ray queue"))) return r;
         }
     }
-    for (int a = 0; a < 3; a++)
-        if ((r = check_cuda(d_sq_[a].alloc(f4), "shadow queue"))) return r;
+    for (int a = 0; a < 2; a++)
+        if ((r = check_cuda(d_sq_[a].alloc(a == 0 ? 2 * f4 : f4), "shadow queue"))) return r;
     if ((r = check_cuda(d_L_.alloc(f4), "path radiance"))) return r;
     if ((r = check_cuda(d_hitd_.alloc(f4), "BSDF-direct hits"))) return r;
     if ((r = check_cuda(d_sort_.alloc(cap * sizeof(int)), "sort index"))) return r;
@@ -997,17 +1007,14 @@ int Session::render_async(int spp) {
     p.sc = scene_view();
     p.dyn = d_dyn_.as<FrameDyn>();
     for (int k = 0; k < 2; k++) {
-        p.q[k].o = d_q_[k][0].as<float4>();
-        p.q[k].d = d_q_[k][1].as<float4>();
-        p.q[k].beta = d_q_[k][2].as<float4>();
-        p.q[k].rng = d_q_[k][3].as<uint2>();
-        p.q[k].hit = d_q_[k][4].as<float4>();
+        p.q[k].od = d_q_[k][0].as<float4>();
+        p.q[k].br = d_q_[k][1].as<float4>();
+        p.q[k].hit = d_q_[k][2].as<float4>();
         p.q[k].hitd = d_hitd_.as<float4>();
-        p.q[k].key = d_q_[k][5].as<int>();
+        p.q[k].key = d_q_[k][3].as<int>();
     }
-    p.sq.o = d_sq_[0].as<float4>();
-    p.sq.d = d_sq_[1].as<float4>();
-    p.sq.c = d_sq_[2].as<float4>();
+    p.sq.od = d_sq_[0].as<float4>();
+    p.sq.c = d_sq_[1].as<float4>();
     p.L = d_L_.as<float4>();
     p.sort_index = d_sort_.as<int>();
     p.ray_index = d_rindex_.as<int>();

@@ -161,13 +161,13 @@ private:
     size_t max_smem_ = 0;
     DevBuf d_qnodes_, d_qfail_;
     int bvh_quant_ = 0;
-    DevBuf d_nodes_, d_prims_, d_tri_p_, d_tri_n_, d_tri_mat_, d_sph_, d_sph_mat_, d_mats_, d_lights_;
+    DevBuf d_nodes_, d_prims_, d_tri_, d_class_, d_sph_, d_sph_mat_, d_mats_, d_lights_;
     DevBuf d_env_rgba_, d_env_marg_, d_env_cond_, d_env_row_, d_env_cut_;
     int build_env_cuts(DevBuf& cuts, const DevBuf& marg, const DevBuf& cond, int w, int h);
     // frame state
     DevBuf d_pass_, d_accum_, d_rgba8_;
-    DevBuf d_q_[2][6];
-    DevBuf d_sq_[3];
+    DevBuf d_q_[2][4];  // ray queues: od, br, hit, key
+    DevBuf d_sq_[2];    // shadow queue: od, c
     DevBuf d_L_, d_hitd_, d_sort_, d_counters_, d_stats_, d_scratch_;
     DevBuf d_rindex_, d_rhist_;  // ray sorting: slot order and bucket counts/cursors
     int queue_cap_ = 0;

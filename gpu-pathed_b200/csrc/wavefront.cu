@@ -166,6 +166,15 @@ __device__ __forceinline__ void camera_path(const FrameParams& p, long long wave
     tag = i | (sid << kTagPathBits);
 }
 
+// A path's random state as the second half of its queue record.
+__device__ __forceinline__ float4 rng_record(uint64_t st) {
+    return make_float4(__uint_as_float((uint32_t)st), __uint_as_float((uint32_t)(st >> 32)), 0.f, 0.f);
+}
+
+__device__ __forceinline__ uint64_t rng_state(float4 r) {
+    return ((uint64_t)__float_as_uint(r.y) << 32) | __float_as_uint(r.x);
+}
+
 // The origin and direction records of queue slot `slot` at `depth` (depth 0 of a wave whose
 // camera rays are not queued: the camera ray of path `slot`, with no MIS pdf).
 template <bool B>
@@ -179,8 +188,9 @@ __device__ __forceinline__ void queue_ray(const FrameParams& p, const PathQueue&
         o4 = make_float4(o.x, o.y, o.z, __int_as_float(tag));
         d4 = make_float4(d.x, d.y, d.z, 0.f);
     } else {
-        o4 = q.o[slot];
-        d4 = q.d[slot];
+        const F8 v = load8(q.od + 2 * (size_t)slot);
+        o4 = v.a;
+        d4 = v.b;
     }
 }
 
@@ -199,10 +209,8 @@ __global__ void k_camera(const __grid_constant__ FrameParams p, long long wave_f
         int tag;
         uint64_t st;
         camera_path<B>(p, wave_first, i, o, d, tag, st);
-        q.o[i] = make_float4(o.x, o.y, o.z, __int_as_float(tag));
-        q.d[i] = make_float4(d.x, d.y, d.z, 0.f);
-        q.beta[i] = make_float4(1.f, 1.f, 1.f, __int_as_float(1));  // camera ray: no MIS
-        q.rng[i] = make_uint2((uint32_t)st, (uint32_t)(st >> 32));
+        store8(q.od + 2 * (size_t)i, make_float4(o.x, o.y, o.z, __int_as_float(tag)), make_float4(d.x, d.y, d.z, 0.f));
+        store8(q.br + 2 * (size_t)i, make_float4(1.f, 1.f, 1.f, __int_as_float(1)), rng_record(st));  // camera ray: no MIS
         p.L[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -228,8 +236,7 @@ __global__ void k_wave_start(const __grid_constant__ FrameParams p, int n) {
 
 __device__ __forceinline__ int material_class(const SceneDevice& sc, int prim) {
     if (prim == kMissPrim) return 0;
-    const int mat = prim >= 0 ? __ldg(sc.tri_mat + prim) : __ldg(sc.sph_mat + ~prim);
-    return sc.mats[mat].type + 1;
+    return __ldg(sc.prim_class + (prim >= 0 ? prim : sc.num_tri + ~prim));
 }
 
 // Warp-sum of per-thread work counters, one 64-bit atomic per warp.
@@ -484,15 +491,11 @@ __device__ __forceinline__ void hit_info(const SceneDevice& sc, V o, V dir, floa
     if (prim >= 0) {
         const float b1 = h4.y, b2 = h4.z;
         const float w0 = 1.f - b1 - b2;
-        const V p0 = mkv(__ldg(sc.tri_p + 3 * prim + 0));
-        const V p1 = mkv(__ldg(sc.tri_p + 3 * prim + 1));
-        const V p2 = mkv(__ldg(sc.tri_p + 3 * prim + 2));
-        const V n0 = mkv(__ldg(sc.tri_n + 3 * prim + 0));
-        const V n1 = mkv(__ldg(sc.tri_n + 3 * prim + 1));
-        const V n2 = mkv(__ldg(sc.tri_n + 3 * prim + 2));
-        point = p0 * w0 + p1 * b1 + p2 * b2;
-        n = w0 * n0 + b1 * n1 + b2 * n2;
-        mat = __ldg(sc.tri_mat + prim);
+        const float4* rec = sc.tri + kTriF4 * prim;
+        const F8 r0 = load8(rec), r1 = load8(rec + 2), r2 = load8(rec + 4);  // p0 p1 | p2 n0 | n1 n2
+        point = mkv(r0.a) * w0 + mkv(r0.b) * b1 + mkv(r1.a) * b2;
+        n = w0 * mkv(r1.b) + b1 * mkv(r2.a) + b2 * mkv(r2.b);
+        mat = __float_as_int(r0.a.w);
     } else {
         const float4 s = __ldg(sc.sph + ~prim);
         point = o + h4.x * dir;
@@ -668,33 +671,37 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
         }
         bool cont_[IPL], shadow_[IPL];
         float4 co_[IPL], cd_[IPL], cb_[IPL], so_[IPL], sd_[IPL], sc_[IPL];
-        uint2 crng_[IPL];
+        uint64_t crng_[IPL];
 #pragma unroll
         for (int item = 0; item < IPL; item++) {
         const int i = base + 32 * item + (threadIdx.x & 31);
         bool cont = false, shadow = false, record = false;
         float4 co, cd, cb, so, sd, sc4;
-        uint2 crng;
+        uint64_t crng;
         GuideRecord rec;
         if (i < count) {
             const int slot = AHEAD ? cur_slot : slot_of(i);
             float4 o4, d4, b4;
             float4 h4 = q.hit[slot];
-            uint2 rng0 = make_uint2(0u, 0u);
+            uint64_t st = 0;
             if (AHEAD && depth == 0) {  // camera ray of path `slot` (p.cam_fused): unit throughput, no MIS
                 V o, d;
                 int tg;
-                uint64_t st0;
-                camera_path<B>(p, wave_first, slot, o, d, tg, st0);
+                camera_path<B>(p, wave_first, slot, o, d, tg, st);
                 o4 = make_float4(o.x, o.y, o.z, __int_as_float(tg));
                 d4 = make_float4(d.x, d.y, d.z, 0.f);
                 b4 = make_float4(1.f, 1.f, 1.f, __int_as_float(1));
-                rng0 = make_uint2((uint32_t)st0, (uint32_t)(st0 >> 32));
             } else {
-                o4 = q.o[slot];
-                d4 = q.d[slot];
-                b4 = q.beta[slot];
-                if (AHEAD) rng0 = q.rng[slot];
+                const F8 od = load8(q.od + 2 * (size_t)slot);
+                o4 = od.a;
+                d4 = od.b;
+                if (AHEAD) {
+                    const F8 br = load8(q.br + 2 * (size_t)slot);
+                    b4 = br.a;
+                    st = rng_state(br.b);
+                } else {
+                    b4 = q.br[2 * (size_t)slot];
+                }
             }
             // a negative t: the BSDF-direct ray stopped closer (hitd), this is the continuation's hit
             const bool split = __float_as_int(h4.x) < 0;
@@ -756,8 +763,7 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
                     const uint32_t pixel =
                         B ? (uint32_t)((gp - p.batch[sid].path_base) / p.batch[sid].spp) : (uint32_t)(gp / p.spp);
                     const uint64_t inc = pcg_inc(pixel);
-                    if (!AHEAD) rng0 = q.rng[slot];
-                    uint64_t st = ((uint64_t)rng0.y << 32) | rng0.x;
+                    if (!AHEAD) st = rng_state(q.br[2 * (size_t)slot + 1]);
                     const bool delta_mat = mtype == kMirror || mtype == kGlass;
                     const bool use_guide = guided && !delta_mat;
                     const float* mix = use_guide ? p.gmix + (size_t)slot * kGuideOut : nullptr;
@@ -833,7 +839,7 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
                             co = make_float4(point.x, point.y, point.z, __int_as_float(tag));
                             cd = make_float4(wworld.x, wworld.y, wworld.z, bs.pdf);
                             cb = make_float4(nb.x, nb.y, nb.z, __int_as_float(bs.delta ? 1 : 0));
-                            crng = make_uint2((uint32_t)st, (uint32_t)(st >> 32));
+                            crng = st;
                             if (GUIDE && p.guide_mode && !delta_mat && ti >= 0 && ti % p.gstride == 0) {
                                 const V wn = normalized(wworld);
                                 const V won = normalized(-dir);
@@ -871,11 +877,9 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
         sc_[item] = sc4;
         }
         if (AHEAD && next_slot >= 0) {
-            prefetch_l2(q.o + next_slot);
-            prefetch_l2(q.d + next_slot);
-            prefetch_l2(q.beta + next_slot);
+            prefetch_l2(q.od + 2 * (size_t)next_slot);
+            prefetch_l2(q.br + 2 * (size_t)next_slot);
             prefetch_l2(q.hit + next_slot);
-            prefetch_l2(q.rng + next_slot);
         }
         int cslot[IPL], sslot[IPL];
         warp_append_pair<IPL>(&p.counters->depth[depth + 1].appended, cont_, cslot, shadow_, sslot);
@@ -883,10 +887,8 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
         for (int item = 0; item < IPL; item++) {
             if (!cont_[item]) continue;
             const int cs = cslot[item];
-            qn.o[cs] = co_[item];
-            qn.d[cs] = cd_[item];
-            qn.beta[cs] = cb_[item];
-            qn.rng[cs] = crng_[item];
+            store8(qn.od + 2 * (size_t)cs, co_[item], cd_[item]);
+            store8(qn.br + 2 * (size_t)cs, cb_[item], rng_record(crng_[item]));
             if (!B && rsort) {
                 const int key = ray_sort_key(p.gframe, co_[item], cd_[item]);
                 qn.key[cs] = key;
@@ -897,8 +899,7 @@ __device__ __forceinline__ void shade_body(const FrameParams& p, int depth, long
         for (int item = 0; item < IPL; item++) {
             if (!shadow_[item]) continue;
             const int ss = sslot[item];
-            p.sq.o[ss] = so_[item];
-            p.sq.d[ss] = sd_[item];
+            store8(p.sq.od + 2 * (size_t)ss, so_[item], sd_[item]);
             p.sq.c[ss] = sc_[item];
         }
         if (AHEAD) {
@@ -987,10 +988,10 @@ __global__ void __maxnreg__(traversal_regs(W)) k_shadow(const __grid_constant__ 
                 const int k = base + __popc(~busy & lanemask_lt());
                 if (slot < 0 && k < count) {
                     slot = k;
-                    const float4 o = p.sq.o[k], d = p.sq.d[k];
-                    r = make_raypre(mkv(o), mkv(d));
-                    tmax = o.w;
-                    tag = __float_as_int(d.w);
+                    const F8 od = load8(p.sq.od + 2 * (size_t)k);
+                    r = make_raypre(mkv(od.a), mkv(od.b));
+                    tmax = od.a.w;
+                    tag = __float_as_int(od.b.w);
                     cur = B ? p.batch[tag_scene(tag)].root : p.sc.root;
                     sp = 0;
                     pend = kEmptyChild;
@@ -1085,7 +1086,7 @@ __global__ void __launch_bounds__(32 * kInferWarps, 2) k_guide_infer(const __gri
         const int slot = grp * 32 + lane;
         float x[kGuideIn];
         if (!B) {
-            if (slot < count) guide_features(p, p.gframe, q.o[slot], q.d[slot], q.hit[slot], x);
+            if (slot < count) guide_features(p, p.gframe, q.od[2 * (size_t)slot], q.od[2 * (size_t)slot + 1], q.hit[slot], x);
             else
                 for (int k = 0; k < kGuideIn; k++) x[k] = 0.f;
             guide_store_input(sx, lane, x);
@@ -1103,8 +1104,8 @@ __global__ void __launch_bounds__(32 * kInferWarps, 2) k_guide_infer(const __gri
             int net = -1, sid = 0;
             float4 o4 = make_float4(0.f, 0.f, 0.f, 0.f), d4 = o4, h4 = o4;
             if (slot < count) {
-                o4 = q.o[slot];
-                d4 = q.d[slot];
+                o4 = q.od[2 * (size_t)slot];
+                d4 = q.od[2 * (size_t)slot + 1];
                 h4 = q.hit[slot];
                 sid = tag_scene(__float_as_int(o4.w));
                 const BatchScene& sb = p.batch[sid];
@@ -1151,7 +1152,7 @@ __global__ void __launch_bounds__(kTcThreads, 2) k_guide_infer_tc(const __grid_c
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const int slot = tile * kTcThreads + t;
         float x[kGuideIn];
-        if (slot < count) guide_features(p, p.gframe, q.o[slot], q.d[slot], q.hit[slot], x);
+        if (slot < count) guide_features(p, p.gframe, q.od[2 * (size_t)slot], q.od[2 * (size_t)slot + 1], q.hit[slot], x);
         else
             for (int k = 0; k < kGuideIn; k++) x[k] = 0.f;
         tc_store_input(s.a[tc_sub()], tc_row(), x);
@@ -1490,9 +1491,9 @@ cudaError_t enqueue_waves(const FrameParams& p_in, const WaveRange* waves, int n
 __device__ __forceinline__ V hit_normal_rn(const SceneDevice& sc, V o, V d, const Hit& h) {
     if (h.prim >= 0) {
         const float w0 = __fsub_rn(__fsub_rn(1.f, h.b1), h.b2);
-        const V n0 = mkv(__ldg(sc.tri_n + 3 * h.prim + 0));
-        const V n1 = mkv(__ldg(sc.tri_n + 3 * h.prim + 1));
-        const V n2 = mkv(__ldg(sc.tri_n + 3 * h.prim + 2));
+        const V n0 = mkv(__ldg(sc.tri + kTriF4 * h.prim + 3));
+        const V n1 = mkv(__ldg(sc.tri + kTriF4 * h.prim + 4));
+        const V n2 = mkv(__ldg(sc.tri + kTriF4 * h.prim + 5));
         return V{__fadd_rn(__fadd_rn(__fmul_rn(w0, n0.x), __fmul_rn(h.b1, n1.x)), __fmul_rn(h.b2, n2.x)),
                  __fadd_rn(__fadd_rn(__fmul_rn(w0, n0.y), __fmul_rn(h.b1, n1.y)), __fmul_rn(h.b2, n2.y)),
                  __fadd_rn(__fadd_rn(__fmul_rn(w0, n0.z), __fmul_rn(h.b1, n1.z)), __fmul_rn(h.b2, n2.z))};
@@ -1686,7 +1687,7 @@ __global__ void __launch_bounds__(kQueryBlock)
             const bool hit = h.prim != kMissPrim, tri = hit && h.prim >= 0;
             out.prim_type[i] = !hit ? -1 : tri ? kTriangle : kSphere;
             out.prim_id[i] = !hit ? -1 : tri ? h.prim : ~h.prim;
-            out.mat_id[i] = !hit ? -1 : tri ? sc.tri_mat[h.prim] : sc.sph_mat[~h.prim];
+            out.mat_id[i] = !hit ? -1 : tri ? __float_as_int(sc.tri[kTriF4 * h.prim].w) : sc.sph_mat[~h.prim];
             out.t[i] = hit ? h.t : 0.f;
             if (out.bary) {
                 out.bary[2 * (size_t)i] = tri ? h.b1 : 0.f;
@@ -1694,6 +1695,26 @@ __global__ void __launch_bounds__(kQueryBlock)
             }
         }
     }
+}
+
+// One thread per triangle: vertices (the material id in p0's fourth word) and normals.
+__global__ void k_pack_triangles(const float* __restrict__ p, const float* __restrict__ n, const int* __restrict__ mat,
+                                 int count, float4* __restrict__ tri) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    const float* a = p + 9 * (size_t)i;
+    const float* b = n + 9 * (size_t)i;
+    float4* o = tri + kTriF4 * (size_t)i;
+    store8(o, make_float4(a[0], a[1], a[2], __int_as_float(mat[i])), make_float4(a[3], a[4], a[5], 0.f));
+    store8(o + 2, make_float4(a[6], a[7], a[8], 0.f), make_float4(b[0], b[1], b[2], 0.f));
+    store8(o + 4, make_float4(b[3], b[4], b[5], 0.f), make_float4(b[6], b[7], b[8], 0.f));
+}
+
+__global__ void k_prim_classes(const __grid_constant__ SceneDevice sc, uint8_t* __restrict__ classes) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= sc.num_tri + sc.num_sph) return;
+    const int mat = i < sc.num_tri ? __float_as_int(sc.tri[kTriF4 * (size_t)i].w) : sc.sph_mat[i - sc.num_tri];
+    classes[i] = (uint8_t)(sc.mats[mat].type + 1);
 }
 
 // One block per CDF; thread k finds cut k.
@@ -1724,7 +1745,7 @@ __global__ void k_hit_test(SceneDevice sc, CameraParams cam, StackShape shape, i
     if (threadIdx.x != 0) return;
     if (of) atomicOr(overflow, 1);
     if (h.prim == kMissPrim) *out = -1;
-    else if (h.prim >= 0) *out = sc.tri_mat[h.prim];
+    else if (h.prim >= 0) *out = __float_as_int(sc.tri[kTriF4 * h.prim].w);
     else *out = sc.sph_mat[~h.prim];
 }
 
@@ -1763,6 +1784,19 @@ cudaError_t enqueue_batch_frame(const FrameParams& p, const WaveRange* waves, in
                            : enqueue_waves<8, false, true>(p, waves, nwaves, stream, marks, side);
         default: return cudaErrorInvalidValue;
     }
+}
+
+cudaError_t pack_triangles(const float* p, const float* n, const int* mat, int count, float4* tri, cudaStream_t stream) {
+    if (count <= 0) return cudaSuccess;
+    k_pack_triangles<<<(count + 255) / 256, 256, 0, stream>>>(p, n, mat, count, tri);
+    return cudaGetLastError();
+}
+
+cudaError_t build_prim_classes(const SceneDevice& sc, uint8_t* classes, cudaStream_t stream) {
+    const int n = sc.num_tri + sc.num_sph;
+    if (n <= 0) return cudaSuccess;
+    k_prim_classes<<<(n + 255) / 256, 256, 0, stream>>>(sc, classes);
+    return cudaGetLastError();
 }
 
 cudaError_t build_cdf_cuts(const float* cdf, int n, int rows, uint16_t* cuts, cudaStream_t stream) {

@@ -9,12 +9,14 @@
 
 namespace pt {
 
-// Per-slot path state of a ray queue (structure of arrays, 16-byte elements).
+// Per-slot path state of a ray queue: 32-byte records, each read or written by one 256-bit access
+// that fills its sector. The shade stage gathers its slots in material order, where 16-byte records
+// moved twice the sectors they used.
 struct PathQueue {
-    float4* o;     // origin.xyz, wave-local path index (int bits)
-    float4* d;     // direction.xyz, pdf of the BSDF sample that produced the ray
-    float4* beta;  // throughput.xyz, flags (int bits): bit 0 = no MIS on the next emission
-    uint2* rng;    // PCG32 state
+    float4* od;    // slot i: [2i] origin.xyz, queue tag; [2i + 1] direction.xyz, pdf of the BSDF sample that
+                   // produced the ray
+    float4* br;    // [2i] throughput.xyz, flags (int bits): bit 0 = no MIS on the next emission;
+                   // [2i + 1] PCG32 state (x, y as bits), unused
     float4* hit;   // t, b1, b2, primitive (int bits); written by the extend stage. A negative t
                    // (-t) marks a continuation hit whose BSDF-direct ray stopped closer (hitd)
     float4* hitd;  // the BSDF-direct ray's hit where it lies closer than the continuation's tMin
@@ -23,9 +25,8 @@ struct PathQueue {
 };
 
 struct ShadowQueue {
-    float4* o;  // origin.xyz, tmax
-    float4* d;  // direction.xyz, wave-local path index (int bits)
-    float4* c;  // contribution (beta * f * cos * Le * w / pdf).xyz, unused
+    float4* od;  // [2i] origin.xyz, tmax; [2i + 1] direction.xyz, queue tag
+    float4* c;   // contribution (beta * f * cos * Le * w / pdf).xyz, unused
 };
 
 constexpr int kMaxDepthLimit = 64;
@@ -252,6 +253,10 @@ cudaError_t enqueue_batch_frame(const FrameParams& p, const WaveRange* waves, in
 cudaError_t enqueue_frame(const FrameParams& p, cudaStream_t stream, StageMarks* marks = nullptr,
                           const SideStream* side = nullptr);
 
+// Triangle records (kTriF4 float4 each) from vertices and normals (9 floats per triangle) and material ids.
+cudaError_t pack_triangles(const float* p, const float* n, const int* mat, int count, float4* tri, cudaStream_t stream);
+// Material classes of every triangle, then of every sphere, of the scene on the device.
+cudaError_t build_prim_classes(const SceneDevice& sc, uint8_t* classes, cudaStream_t stream);
 // Cut points (kCdfCuts + 1 per row) of `rows` CDFs of n <= kCdfCutMax values each.
 cudaError_t build_cdf_cuts(const float* cdf, int n, int rows, uint16_t* cuts, cudaStream_t stream);
 
