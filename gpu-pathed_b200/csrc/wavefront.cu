@@ -427,60 +427,93 @@ __global__ void __maxnreg__(traversal_regs(W)) k_extend(const __grid_constant__ 
     if (CNT) flush_work(work, &p.stats->extend_nodes, &p.stats->extend_prims);
 }
 
-constexpr int kSortItems = 4;  // queue entries per thread and chunk of the material sort
-__global__ void k_sort(const __grid_constant__ FrameParams p, int depth) {
+// Material sort: a stable counting sort of the queue's slots by class. A block takes chunks of
+// kSortChunk slots, kSortItems consecutive ones per thread; counts of the eight classes (7: no slot)
+// travel as 16-bit fields of two 64-bit words, so one warp scan ranks a warp's 256 slots, and one
+// atomic per class and chunk reserves the chunk's places. The chunk's sorted slots are gathered in
+// shared memory and written out in runs. Keeping slot order within a class keeps the shade stage's
+// gathers near each other: 4096-slot chunks written unstaged, strided over the threads, cost the
+// spheres 1.8%. Sort stage before (one slot per lane ranked at a time by match.any, 107 instructions per
+// slot) -> now, per frame: spheres 0.87 -> 0.66 ms, batch of six 0.33 -> 0.28.
+constexpr int kSortBlock = 256, kSortItems = 8, kSortChunk = kSortBlock * kSortItems;
+__device__ __forceinline__ unsigned long long class_one(int cls) { return 1ull << (16 * (cls & 3)); }
+__device__ __forceinline__ int class_field(unsigned long long lo, unsigned long long hi, int cls) {
+    return (int)(((cls < 4 ? lo : hi) >> (16 * (cls & 3))) & 0xffffu);
+}
+__global__ void __launch_bounds__(kSortBlock) k_sort(const __grid_constant__ FrameParams p, int depth) {
+    __shared__ unsigned long long s_tot[kSortBlock / 32][2];  // per warp: counts of classes 0-3, 4-7
+    __shared__ int s_local[9], s_shift[8];  // where a class begins in the chunk; its place in the order, less that
+    __shared__ int s_slot[kSortChunk];
     const int count = ray_count(p, depth);
-    const PathQueue q = p.q[depth & 1];
-    int off[kMaterialClasses];
-    int acc = 0;
+    const int* __restrict__ keys = p.q[depth & 1].key;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    int first = 0;  // threads 0-6: where class t begins in the whole order
+    if (t < kMaterialClasses)
+        for (int c = 0; c < t; c++) first += p.counters->depth[depth].sort_count[c];
+    for (int base = blockIdx.x * kSortChunk; base < count; base += gridDim.x * kSortChunk) {
+        const int i0 = base + kSortItems * t;
+        int key[kSortItems];
 #pragma unroll
-    for (int c = 0; c < kMaterialClasses; c++) {
-        off[c] = acc;
-        acc += p.counters->depth[depth].sort_count[c];
-    }
-    // Slots are reserved per block and chunk of kSortItems x blockDim.x entries: warps add
-    // their class counts into shared counters, then one global atomic per class and chunk
-    // reserves the chunk's range (the grid is capped at a few blocks per SM and strides over
-    // the queue). Several entries per thread share each chunk's barriers and atomics.
-    __shared__ int s_cnt[8], s_base[8];
-    const int stride = gridDim.x * blockDim.x * kSortItems;
-    const int lane = threadIdx.x & 31;
-    const unsigned lt = lanemask_lt();
-    for (int base = blockIdx.x * blockDim.x * kSortItems; base < count; base += stride) {
-        if (threadIdx.x < 8) s_cnt[threadIdx.x] = 0;
-        __syncthreads();
-        int key[kSortItems], b[kSortItems], leader[kSortItems];
-        unsigned peers[kSortItems];
+        for (int j = 0; j < kSortItems; j += 4) {
+            if (i0 + j + 3 < count) {
+                const int4 v = *reinterpret_cast<const int4*>(keys + i0 + j);
+                key[j] = v.x; key[j + 1] = v.y; key[j + 2] = v.z; key[j + 3] = v.w;
+            } else {
 #pragma unroll
-        for (int j = 0; j < kSortItems; j++) {
-            const int i = base + j * blockDim.x + threadIdx.x;
-            key[j] = i < count ? q.key[i] : 7;  // 7: no entry (no class uses it)
-        }
-#pragma unroll
-        for (int j = 0; j < kSortItems; j++) {
-            const int i = base + j * blockDim.x + threadIdx.x;
-            peers[j] = __match_any_sync(0xffffffffu, key[j]);
-            leader[j] = __ffs(peers[j]) - 1;
-            b[j] = 0;
-            if (i < count && lane == leader[j]) b[j] = atomicAdd(&s_cnt[key[j]], __popc(peers[j]));
-        }
-        __syncthreads();
-        if (threadIdx.x < kMaterialClasses && s_cnt[threadIdx.x] > 0)
-            s_base[threadIdx.x] = atomicAdd(&p.counters->depth[depth].sort_fill[threadIdx.x], s_cnt[threadIdx.x]);
-        __syncthreads();
-#pragma unroll
-        for (int j = 0; j < kSortItems; j++) {
-            const int i = base + j * blockDim.x + threadIdx.x;
-            const int bj = __shfl_sync(0xffffffffu, b[j], leader[j]);
-            if (i < count) {
-                int ko = 0;
-#pragma unroll
-                for (int c = 0; c < kMaterialClasses; c++)
-                    if (c == key[j]) ko = off[c] + s_base[c];
-                p.sort_index[ko + bj + __popc(peers[j] & lt)] = i;
+                for (int k = 0; k < 4; k++) key[j + k] = i0 + j + k < count ? keys[i0 + j + k] : 7;
             }
         }
-        __syncthreads();  // s_cnt / s_base are reused by the next chunk
+        unsigned long long lo = 0, hi = 0;
+#pragma unroll
+        for (int j = 0; j < kSortItems; j++) {
+            if (key[j] < 4) lo += class_one(key[j]);
+            else hi += class_one(key[j]);
+        }
+        unsigned long long xlo = lo, xhi = hi;  // inclusive scan over the warp
+#pragma unroll
+        for (int k = 1; k < 32; k <<= 1) {
+            const unsigned long long ylo = __shfl_up_sync(0xffffffffu, xlo, k);
+            const unsigned long long yhi = __shfl_up_sync(0xffffffffu, xhi, k);
+            if (lane >= k) { xlo += ylo; xhi += yhi; }
+        }
+        if (lane == 31) { s_tot[warp][0] = xlo; s_tot[warp][1] = xhi; }
+        __syncthreads();
+        unsigned long long blo = 0, bhi = 0, plo = 0, phi = 0;  // the block's totals; those of the warps before
+#pragma unroll
+        for (int w = 0; w < kSortBlock / 32; w++) {
+            if (w == warp) { plo = blo; phi = bhi; }
+            blo += s_tot[w][0];
+            bhi += s_tot[w][1];
+        }
+        if (t < 8) {
+            int at = 0;
+            for (int c = 0; c < t; c++) at += class_field(blo, bhi, c);
+            const int n = class_field(blo, bhi, t);
+            s_local[t] = at;
+            if (t < kMaterialClasses && n > 0)
+                s_shift[t] = first + atomicAdd(&p.counters->depth[depth].sort_fill[t], n) - at;
+        }
+        __syncthreads();
+        plo += xlo - lo;
+        phi += xhi - hi;  // slots of each class before this thread's
+#pragma unroll
+        for (int j = 0; j < kSortItems; j++) {
+            const int c = key[j];
+            s_slot[s_local[c] + class_field(plo, phi, c)] = (c << 28) | (kSortItems * t + j);
+            if (c < 4) plo += class_one(c);
+            else phi += class_one(c);
+        }
+        __syncthreads();
+        const int n = min(kSortChunk, count - base);
+#pragma unroll
+        for (int j = 0; j < kSortItems; j++) {
+            const int k = j * kSortBlock + t;
+            if (k < n) {
+                const unsigned v = (unsigned)s_slot[k];
+                p.sort_index[s_shift[v >> 28] + k] = base + (int)(v & 0xfffffffu);
+            }
+        }
+        __syncthreads();  // the next chunk reuses the shared arrays
     }
 }
 
@@ -1424,8 +1457,7 @@ cudaError_t enqueue_waves(const FrameParams& p_in, const WaveRange* waves, int n
             extend<<<grid_e, p.shape.block_extend, smem_e, stream>>>(p, d, wave_first);
             mark(kStageExtend);
             if (p.shape.sort_materials) {
-                k_sort<<<std::min((n + 256 * kSortItems - 1) / (256 * kSortItems), p.num_sms * 8), 256, 0, stream>>>(
-                    p, d);
+                k_sort<<<std::min((n + kSortChunk - 1) / kSortChunk, p.num_sms * 8), kSortBlock, 0, stream>>>(p, d);
                 mark(kStageSort);
             }
             if (p.guide_mode == 2 && d < p.max_depth - 1) {
