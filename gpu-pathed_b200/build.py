@@ -30,7 +30,7 @@ CU_SOURCES = ["wavefront.cu", "guide.cu", "bvh_gpu.cu", "probe.cu"]
 # differently in each instantiation), at about 2% of the shade stage's time.
 CU_FLAGS = {"wavefront.cu": ["-fmad=false"]}
 CPP_SOURCES = ["host_scene.cpp", "bvh_build.cpp", "host_util.cpp", "assets.cpp", "session.cpp", "session_batch.cpp",
-               "capi.cpp"]
+               "session_query.cpp", "capi.cpp"]
 HEADERS = [f for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))] if os.path.isdir(CSRC) else []
 
 

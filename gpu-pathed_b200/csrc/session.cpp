@@ -1663,41 +1663,7 @@ int Session::trace_rays(const float* o, const float* d, const float* tmin, const
         if (hof) return fail(PT_ERR_DEVICE, "traversal stack overflow reported by a kernel");
         return PT_OK;
     }
-    // inputs 3+3+1+1 floats, outputs 3 ints + t + 2 bary, plus the overflow flag
-    const size_t N = (size_t)n;
-    const size_t bytes = N * 4 * (8 + 6) + 256;
-    if ((r = check_cuda(d_scratch_.alloc(bytes), "scratch"))) return r;
-    char* base = d_scratch_.as<char>();
-    float* dO = (float*)base;
-    float* dD = dO + 3 * N;
-    float* dTmin = dD + 3 * N;
-    float* dTmax = dTmin + N;
-    int* dPt = (int*)(dTmax + N);
-    int* dPid = dPt + N;
-    int* dMid = dPid + N;
-    float* dT = (float*)(dMid + N);
-    float* dB = dT + N;
-    int* dOf = (int*)(dB + 2 * N);
-    cudaStream_t st = stream_;
-    if ((r = check_cuda(cudaMemcpyAsync(dO, o, 12 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
-    if ((r = check_cuda(cudaMemcpyAsync(dD, d, 12 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
-    if ((r = check_cuda(cudaMemcpyAsync(dTmin, tmin, 4 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
-    if ((r = check_cuda(cudaMemcpyAsync(dTmax, tmax, 4 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
-    if ((r = check_cuda(cudaMemsetAsync(dOf, 0, 8, st), "memset"))) return r;
-    if ((r = check_cuda(enqueue_trace_rays(scene_view(), sd, dO, dD, dTmin, dTmax, n, dPt, dPid, dMid, dT,
-                                           bary ? dB : nullptr, dOf, st),
-                        "trace rays")))
-        return r;
-    if ((r = check_cuda(cudaMemcpyAsync(pty, dPt, 4 * N, cudaMemcpyDeviceToHost, st), "copy hits"))) return r;
-    if ((r = check_cuda(cudaMemcpyAsync(pid, dPid, 4 * N, cudaMemcpyDeviceToHost, st), "copy hits"))) return r;
-    if ((r = check_cuda(cudaMemcpyAsync(mid, dMid, 4 * N, cudaMemcpyDeviceToHost, st), "copy hits"))) return r;
-    if ((r = check_cuda(cudaMemcpyAsync(t, dT, 4 * N, cudaMemcpyDeviceToHost, st), "copy hits"))) return r;
-    if (bary && (r = check_cuda(cudaMemcpyAsync(bary, dB, 8 * N, cudaMemcpyDeviceToHost, st), "copy hits"))) return r;
-    int hof = 0;
-    if ((r = check_cuda(cudaMemcpyAsync(&hof, dOf, 4, cudaMemcpyDeviceToHost, st), "copy flag"))) return r;
-    if ((r = check_cuda(cudaStreamSynchronize(st), "trace rays"))) return r;
-    if (hof) return fail(PT_ERR_DEVICE, "traversal stack overflow reported by a kernel");
-    return PT_OK;
+    return host_query(HostRays{o, d, tmin, tmax, n}, HostHits{pty, pid, mid, t, bary, nullptr});
 }
 
 int Session::trace_rays_static(const float* o, const float* d, const float* tmin, const float* tmax, int n, int* pty,
@@ -1739,28 +1705,7 @@ int Session::occluded(const float* o, const float* d, const float* tmin, const f
     if (in_flight_ && (r = wait(nullptr))) return r;
     if (scene_dirty_ && (r = upload_scene())) return r;
     if (mats_dirty_ && (r = upload_materials())) return r;
-    const StackShape sd = stack_shape(d_spill_, num_sms_ * kSmThreads);
-    const size_t N = (size_t)n;
-    if ((r = check_cuda(d_scratch_.alloc(N * 4 * 9 + 256), "scratch"))) return r;
-    float* dO = d_scratch_.as<float>();
-    float* dD = dO + 3 * N;
-    float* dTmin = dD + 3 * N;
-    float* dTmax = dTmin + N;
-    int* dOcc = (int*)(dTmax + N);
-    int* dOf = dOcc + N;
-    cudaStream_t st = stream_;
-    if ((r = check_cuda(cudaMemcpyAsync(dO, o, 12 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
-    if ((r = check_cuda(cudaMemcpyAsync(dD, d, 12 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
-    if ((r = check_cuda(cudaMemcpyAsync(dTmin, tmin, 4 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
-    if ((r = check_cuda(cudaMemcpyAsync(dTmax, tmax, 4 * N, cudaMemcpyHostToDevice, st), "copy rays"))) return r;
-    if ((r = check_cuda(cudaMemsetAsync(dOf, 0, 8, st), "memset"))) return r;
-    if ((r = check_cuda(enqueue_occluded(scene_view(), sd, dO, dD, dTmin, dTmax, n, dOcc, dOf, st), "occluded"))) return r;
-    if ((r = check_cuda(cudaMemcpyAsync(occ, dOcc, 4 * N, cudaMemcpyDeviceToHost, st), "copy"))) return r;
-    int hof = 0;
-    if ((r = check_cuda(cudaMemcpyAsync(&hof, dOf, 4, cudaMemcpyDeviceToHost, st), "copy flag"))) return r;
-    if ((r = check_cuda(cudaStreamSynchronize(st), "occluded"))) return r;
-    if (hof) return fail(PT_ERR_DEVICE, "traversal stack overflow reported by a kernel");
-    return PT_OK;
+    return host_query(HostRays{o, d, tmin, tmax, n}, HostHits{nullptr, nullptr, nullptr, nullptr, nullptr, occ});
 }
 
 }  // namespace pt

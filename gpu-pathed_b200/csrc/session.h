@@ -45,6 +45,29 @@ cudaError_t upload(DevBuf& b, const std::vector<T>& v, cudaStream_t st) {
     return cudaMemcpyAsync(b.p, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, st);
 }
 
+// Host-array queries: the caller's rays and results, and their staging (session_query.cpp).
+struct HostRays {
+    const float *o, *d, *tmin, *tmax;
+    int n;
+};
+struct HostHits {  // closest hit: the five arrays (bary may be null); any hit: occluded alone
+    int *prim_type, *prim_id, *mat_id;
+    float *t, *bary;
+    int* occluded;
+};
+constexpr int kQueryWorkers = 8;
+struct QueryStaging {  // one chunk of page-locked and device memory and a stream per worker
+    void* host = nullptr;
+    size_t host_bytes = 0;
+    DevBuf dev;
+    std::vector<cudaStream_t> streams;
+    QueryStaging() = default;
+    QueryStaging(const QueryStaging&) = delete;
+    QueryStaging& operator=(const QueryStaging&) = delete;
+    ~QueryStaging();
+    cudaError_t ensure(int workers, size_t bytes_each);
+};
+
 inline bool env_cuts_fit(int w, int h) { return w <= kCdfCutMax && h <= kCdfCutMax; }
 inline void set_env_cuts(EnvDevice& e, const DevBuf& cuts, int w, int h) {
     e.marg_cut = env_cuts_fit(w, h) ? cuts.as<uint16_t>() : nullptr;
@@ -320,6 +343,8 @@ private:
     // stream_, the shadow stage beside it, and the allocation-free queries on query_stream_
     DevBuf d_spill_, d_shadow_spill_, d_query_spill_;
     int ensure_stacks();
+    QueryStaging query_;
+    int host_query(const HostRays& rays, const HostHits& out);
     StackShape stack_shape(const DevBuf& spill, int threads) const;
 };
 

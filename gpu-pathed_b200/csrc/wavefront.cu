@@ -1712,7 +1712,7 @@ __global__ void __launch_bounds__(kQueryBlock)
         traverse_round<W, ANY, false>(sc.nodes, sc.prims, quant, false, r, tmin, tmax, st, h, cur, pend, sp, alive, occ,
                                       of, nullptr, wt);
         if (!was || alive) continue;
-        if (of) atomicOr(flags, 1);
+        if (of) *flags = 1;  // every writer stores the same value
         if (ANY) {
             out.occluded[i] = occ ? 1 : 0;
         } else {

@@ -64,3 +64,21 @@ def test_query_counts(n):
         assert np.array_equal(g[k], np.concatenate([p[k] for p in parts])), k
     assert np.array_equal(occ, (g["prim_type"] >= 0).astype(np.int32))
     s.close()
+
+
+@pytest.mark.gpu
+def test_query_arrays_may_overlap():
+    """results written over rays (a call of several chunks): every ray is read first"""
+    n = 70001
+    s = pathed.Session(32, 32)
+    s.load_config(0)
+    o, d, tmin, tmax = seeded_rays(s.export_scene(), n, seed=9)
+    ref = s.trace_rays(o, d, tmin, tmax)
+    out = [np.empty(n, np.int32) for _ in range(3)]
+    t = o.reshape(-1)[n:]  # the distances go over the origins' later two thirds
+    s._check(pathed.lib.pt_trace_rays(s._h, o.ctypes.data, d.ctypes.data, tmin.ctypes.data, tmax.ctypes.data, n,
+                                      out[0].ctypes.data, out[1].ctypes.data, out[2].ctypes.data, t.ctypes.data, None))
+    for k, got in zip(("prim_type", "prim_id", "mat_id"), out):
+        assert np.array_equal(got, ref[k]), k
+    assert np.array_equal(t[:n], ref["t"])
+    s.close()
