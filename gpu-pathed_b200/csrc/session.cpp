@@ -76,6 +76,7 @@ Session::~Session() {
             cudaStreamDestroy(query_stream_);
         }
         if (h_stats_) cudaFreeHost(h_stats_);
+        if (h_pick_) cudaFreeHost(h_pick_);
     }
 }
 
@@ -141,6 +142,7 @@ int Session::ensure_device() {
                        cls_done_.data()};
     if ((r = check_cuda(cudaMallocHost((void**)&h_stats_, sizeof(FrameStats)), "cudaMallocHost"))) return r;
     std::memset(h_stats_, 0, sizeof(FrameStats));
+    if ((r = check_cuda(cudaMallocHost((void**)&h_pick_, 2 * sizeof(int)), "cudaMallocHost"))) return r;
     if ((r = check_cuda(d_counters_.alloc(sizeof(WaveCounters)), "counters"))) return r;
     if ((r = check_cuda(d_stats_.alloc(sizeof(FrameStats)), "stats"))) return r;
     if ((r = check_cuda(d_dyn_.alloc(sizeof(FrameDyn)), "frame constants"))) return r;
@@ -1620,16 +1622,13 @@ int Session::hit_test(int x, int y, int* mat) {
     if (mats_dirty_ && (r = upload_materials())) return r;
     std::string err;
     if (!make_camera(camspec_, w_, h_, cam_, err)) return fail(PT_ERR_ARG, err);
-    if ((r = check_cuda(d_scratch_.alloc(64), "scratch"))) return r;
-    int* dm = d_scratch_.as<int>();
-    if ((r = check_cuda(cudaMemsetAsync(dm, 0, 8, stream_), "memset"))) return r;
     StackShape stack = stack_shape(d_spill_, 32);  // one query: all of its entries in shared memory
     stack.shared = stack.cap = stack_need(bvh_.width, bvh_.depth);
-    if ((r = check_cuda(enqueue_hit_test(scene_view(), cam_, stack, x, y, dm, dm + 1, stream_), "hit test")))
+    // the kernel writes the material and the overflow flag to page-locked memory: one launch, no copies
+    if ((r = check_cuda(enqueue_hit_test(scene_view(), cam_, stack, x, y, h_pick_, h_pick_ + 1, stream_), "hit test")))
         return r;
-    int res[2];
-    if ((r = check_cuda(cudaMemcpyAsync(res, dm, 8, cudaMemcpyDeviceToHost, stream_), "hit test readback"))) return r;
     if ((r = check_cuda(cudaStreamSynchronize(stream_), "hit test"))) return r;
+    const int res[2] = {h_pick_[0], h_pick_[1]};
     if (res[1]) return fail(PT_ERR_DEVICE, "traversal stack overflow reported by a kernel");
     *mat = res[0];
     return PT_OK;

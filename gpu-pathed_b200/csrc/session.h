@@ -219,6 +219,7 @@ private:
     int frames_ = 0;
     FrameStats last_stats_{};
     FrameStats* h_stats_ = nullptr;  // pinned
+    int* h_pick_ = nullptr;          // pinned: a hit test's material and overflow flag
     // profiling
     int stage_timing_ = 0;
     int work_counters_ = 0;

@@ -1775,7 +1775,7 @@ __global__ void k_hit_test(SceneDevice sc, CameraParams cam, StackShape shape, i
     // the whole warp enters the traversal; lane 0 carries the query and owns the stack
     traverse<W, false>(sc, r, 0.f, FLT_MAX, threadIdx.x == 0, LaneStack<false>{stk, 1, shape}, h, of);
     if (threadIdx.x != 0) return;
-    if (of) atomicOr(overflow, 1);
+    *overflow = of ? 1 : 0;
     if (h.prim == kMissPrim) *out = -1;
     else if (h.prim >= 0) *out = __float_as_int(sc.tri[kTriF4 * h.prim].w);
     else *out = sc.sph_mat[~h.prim];
