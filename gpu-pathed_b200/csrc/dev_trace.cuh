@@ -423,14 +423,15 @@ struct LaneStack {
 // drops none). So are empty children: a ray whose direction is NaN or infinite on all axes finds
 // every slab open, an empty child's too.
 template <bool ANY>
-__device__ __forceinline__ int stack_pop(const LaneStack<ANY>& st, float tmax, const Hit& best, int& sp) {
+__device__ __forceinline__ int stack_pop(const LaneStack<ANY>& st, float tmax, const Hit& best, int& sp,
+                                         int bottom = 0) {
     if constexpr (ANY) {
-        if (sp == 0) return kEmptyChild;
+        if (sp == bottom) return kEmptyChild;
         sp--;
         return *st.slot(sp);
     } else {
         const float thr = (best.prim == kMissPrim ? tmax : best.t) * kBoxSlack * kBoxSlack;
-        while (sp > 0) {
+        while (sp > bottom) {
             sp--;
             const int2 e = *st.slot(sp);
             if (!(__int_as_float(e.y) > thr) && e.x != kEmptyChild) return e.x;
@@ -447,7 +448,8 @@ __device__ __forceinline__ int stack_pop(const LaneStack<ANY>& st, float tmax, c
 template <int W, bool ANY, bool CNT>
 __device__ __forceinline__ void node_step(const float4* __restrict__ nodes, bool quant, const RayPre& r, float tmin,
                                           float tmax, const LaneStack<ANY>& st, const Hit& best, int& cur, int& sp,
-                                          bool& alive, int& overflow, TraceWork* work, bool near = false) {
+                                          bool& alive, int& overflow, TraceWork* work, bool near = false,
+                                          int bottom = 0) {
     constexpr int kNF4 = sizeof(BvhNode<W>) / 16;
     const float inf = __int_as_float(0x7f800000);
     NodeView<W> nv;
@@ -493,7 +495,7 @@ __device__ __forceinline__ void node_step(const float4* __restrict__ nodes, bool
             overflow = 1;
             alive = false;  // reported to the host; the query gives up
         } else if (next == kEmptyChild) {
-            next = stack_pop<ANY>(st, tmax, best, sp);
+            next = stack_pop<ANY>(st, tmax, best, sp, bottom);
             if (next == kEmptyChild) alive = false;
         }
         cur = next;
@@ -527,7 +529,7 @@ __device__ __forceinline__ void node_step(const float4* __restrict__ nodes, bool
         overflow = 1;
         alive = false;  // reported to the host; the query gives up
     } else if (next == kEmptyChild) {
-        next = stack_pop<ANY>(st, tmax, best, sp);
+        next = stack_pop<ANY>(st, tmax, best, sp, bottom);
         if (next == kEmptyChild) alive = false;
     }
     cur = next;
@@ -557,11 +559,11 @@ __device__ __forceinline__ void leaf_test(const float4* __restrict__ prims, int 
 template <bool ANY, bool CNT>
 __device__ __forceinline__ void leaf_step(const float4* __restrict__ prims, const RayPre& r, float tmin, float tmax,
                                           const LaneStack<ANY>& st, Hit& best, int& cur, int& sp, bool& alive,
-                                          bool& hit_any, TraceWork* work, bool wt) {
+                                          bool& hit_any, TraceWork* work, bool wt, int bottom) {
     leaf_test<ANY, CNT>(prims, cur, r, tmin, tmax, best, hit_any, work, wt);
     if (ANY && hit_any) alive = false;
     if (alive) {
-        cur = stack_pop<ANY>(st, tmax, best, sp);
+        cur = stack_pop<ANY>(st, tmax, best, sp, bottom);
         if (cur == kEmptyChild) alive = false;
     }
 }
@@ -581,14 +583,14 @@ __device__ __forceinline__ void traverse_round(const float4* __restrict__ nodes,
                                                bool quant, bool spec, const RayPre& r, float tmin, float tmax,
                                                const LaneStack<ANY>& st, Hit& best, int& cur, int& pend, int& sp,
                                                bool& alive, bool& hit_any, int& overflow, TraceWork* work,
-                                               bool wt = false, bool near = false) {
+                                               bool wt = false, bool near = false, int bottom = 0) {
     // ---- phase 1: internal nodes, while enough live lanes have found no leaf
     const int live = __popc(__ballot_sync(0xffffffffu, alive));
     for (;;) {
         const int searching = __popc(__ballot_sync(0xffffffffu, alive && cur >= 0 && pend == kEmptyChild));
         if (3 * searching <= live) break;
         if (alive && cur >= 0) {
-            node_step<W, ANY, CNT>(nodes, quant, r, tmin, tmax, st, best, cur, sp, alive, overflow, work, near);
+            node_step<W, ANY, CNT>(nodes, quant, r, tmin, tmax, st, best, cur, sp, alive, overflow, work, near, bottom);
             if (spec) {
                 if (!alive && !overflow && pend != kEmptyChild) {
                     alive = true;  // the stack ran empty: only the parked leaf is left
@@ -596,7 +598,7 @@ __device__ __forceinline__ void traverse_round(const float4* __restrict__ nodes,
                     pend = kEmptyChild;
                 } else if (alive && cur < 0 && pend == kEmptyChild) {
                     pend = cur;  // park the first leaf and keep descending
-                    cur = stack_pop<ANY>(st, tmax, best, sp);
+                    cur = stack_pop<ANY>(st, tmax, best, sp, bottom);
                     if (cur == kEmptyChild) {
                         cur = pend;
                         pend = kEmptyChild;
@@ -612,7 +614,130 @@ __device__ __forceinline__ void traverse_round(const float4* __restrict__ nodes,
         if (ANY && hit_any) alive = false;
     }
     if (alive && cur < 0)
-        leaf_step<ANY, CNT>(prims, r, tmin, tmax, st, best, cur, sp, alive, hit_any, work, wt);
+        leaf_step<ANY, CNT>(prims, r, tmin, tmax, st, best, cur, sp, alive, hit_any, work, wt, bottom);
+}
+
+__device__ __forceinline__ unsigned lanemask_lt() {
+    unsigned m;
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
+    return m;
+}
+// Position of the k-th set bit (k from 0, below the mask's count).
+__device__ __forceinline__ int nth_bit(unsigned mask, int k) {
+    int pos = 0;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1) {
+        const int c = __popc(mask & ((1u << s) - 1u));
+        if (k >= c) {
+            k -= c;
+            pos += s;
+            mask >>= s;
+        }
+    }
+    return pos;
+}
+// The better of two closest hits of one query (the total order of leaf_entry).
+__device__ __forceinline__ void merge_hit(Hit& best, const Hit& c) {
+    if (c.prim == kMissPrim) return;
+    const bool tie = c.prim >= 0 ? (best.prim < 0 || c.prim > best.prim) : (best.prim < 0 && c.prim > best.prim);
+    if (best.prim == kMissPrim || c.t < best.t || (c.t == best.t && tie)) best = c;
+}
+__device__ __forceinline__ float shfl_f(float v, int lane) { return __shfl_sync(0xffffffffu, v, lane); }
+
+// The end of a persistent traversal: the queue is empty and few lanes of the warp still carry a query.
+// Their queries are the long ones (on the meshes a launch ran on for 50 to 200 us after half of its warps
+// had ended), so the idle lanes help: each takes the bottom entry of a busy lane's stack, the
+// largest subtree left behind, with the ray, and traverses it as its own. A helper's hit is
+// merged into its owner's when the helper runs dry (closest hits are the minimum of a total order, so the
+// split changes nothing); helpers cull against the owner's hit as of the last round, one ulp
+// farther, so that ties still reach the merge. A query ends when its owner and all of its helpers
+// have. `has`: the lane carries a query; `end()` finishes the lane's query and returns whether it
+// started another (with cur, sp, h, tmin set and alive true).
+template <int W, bool ANY, bool CNT, class End>
+__device__ __forceinline__ void traverse_tail(const float4* __restrict__ nodes, const float4* __restrict__ prims,
+                                              bool quant, RayPre& r, float& tmin, float& tmax,
+                                              const LaneStack<ANY>& st, Hit& h, int& cur, int& sp, bool& alive,
+                                              bool& occ, int& of, bool has, TraceWork* work, bool wt, bool near,
+                                              End&& end) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const float full = tmax;       // this lane's own query's bound
+    int owner = has ? lane : -1;   // the lane whose query this lane works on
+    int bottom = 0, pend = kEmptyChild;
+    // a ray that is not finite is not shared: its hits can be NaN, and the last one visited stands
+    const bool shares = isfinite(r.ix + r.iy + r.iz + r.ox + r.oy + r.oz);
+    while (__any_sync(kAll, owner >= 0)) {
+        const unsigned idle = __ballot_sync(kAll, owner < 0);
+        const unsigned rich = __ballot_sync(kAll, alive && sp - bottom >= 2 && (shares || owner != lane));
+        if (idle != 0 && rich != 0) {
+            const int n = min(__popc(idle), __popc(rich));
+            const int rank = __popc((owner < 0 ? idle : rich) & lanemask_lt());
+            const bool take = owner < 0 && rank < n;
+            const bool give = ((rich >> lane) & 1u) && rank < n;
+            const int from = take ? nth_bit(rich, rank) : lane;
+            int child = kEmptyChild;
+            if (give) {
+                if constexpr (ANY) child = *st.slot(bottom);
+                else child = st.slot(bottom)->x;
+                bottom++;
+            }
+            child = __shfl_sync(kAll, child, from);
+            const float bound = ANY || h.prim == kMissPrim ? tmax : __int_as_float(__float_as_int(fmaxf(h.t, 0.f)) + 1);
+            const float lim = shfl_f(bound, from), t0 = shfl_f(tmin, from);
+            const int of_query = __shfl_sync(kAll, owner, from);
+            RayPre v;
+            v.o = V{shfl_f(r.o.x, from), shfl_f(r.o.y, from), shfl_f(r.o.z, from)};
+            v.d = V{shfl_f(r.d.x, from), shfl_f(r.d.y, from), shfl_f(r.d.z, from)};
+            v.ix = shfl_f(r.ix, from); v.iy = shfl_f(r.iy, from); v.iz = shfl_f(r.iz, from);
+            v.ox = shfl_f(r.ox, from); v.oy = shfl_f(r.oy, from); v.oz = shfl_f(r.oz, from);
+            if (take) {
+                r = v;
+                tmin = t0;
+                tmax = lim;
+                owner = of_query;
+                h = Hit{lim, 0.f, 0.f, kMissPrim};
+                cur = child;
+                sp = bottom = 0;
+                occ = false;
+                of = 0;
+                alive = child != kEmptyChild;
+            }
+        }
+        traverse_round<W, ANY, CNT>(nodes, prims, quant, false, r, tmin, tmax, st, h, cur, pend, sp, alive, occ, of,
+                                    work, wt, near, bottom);
+        // the lanes of one query
+        const unsigned group = __match_any_sync(kAll, owner >= 0 ? owner : 32 + lane);
+        const unsigned failed = __ballot_sync(kAll, owner >= 0 && of != 0);
+        const unsigned hits = __ballot_sync(kAll, ANY && owner >= 0 && occ);
+        if ((failed | hits) & group) {  // a query gives up, or is occluded, as a whole
+            if (failed & group) of = 1;
+            if (hits & group) occ = true;
+            alive = false;
+        }
+        const bool helper = owner >= 0 && owner != lane;
+        if constexpr (!ANY) {
+            unsigned done = __ballot_sync(kAll, helper && !alive);
+            while (done) {
+                const int b = __ffs(done) - 1;
+                done &= done - 1;
+                const Hit c{shfl_f(h.t, b), shfl_f(h.b1, b), shfl_f(h.b2, b), __shfl_sync(kAll, h.prim, b)};
+                if (lane == __shfl_sync(kAll, owner, b)) merge_hit(h, c);
+            }
+            const float bound = h.prim == kMissPrim ? tmax : __int_as_float(__float_as_int(fmaxf(h.t, 0.f)) + 1);
+            const float lim = shfl_f(bound, owner >= 0 ? owner : lane);
+            if (helper && lim < tmax) {
+                tmax = lim;
+                if (h.prim != kMissPrim && h.t > lim) h.prim = kMissPrim;
+            }
+        }
+        const unsigned live = __ballot_sync(kAll, alive);
+        if (helper && !alive) owner = -1;
+        if (owner == lane && !(live & group)) {
+            tmax = full;
+            bottom = 0;
+            if (!end()) owner = -1;
+        }
+    }
 }
 
 // Warp-synchronous traversal: every lane of the warp calls this together (`active` marks the

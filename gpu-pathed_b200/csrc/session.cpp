@@ -864,6 +864,8 @@ StackShape Session::stack_shape(const DevBuf& spill, int threads) const {
     st.shared = std::min(need, kStackShared);
     st.cap = test_stack_cap_ > 0 ? std::min(test_stack_cap_, need) : need;
     st.spill_stride = threads;
+    // frames that count work keep each query on its own lane: the counts are the queries' own visits
+    st.tail = bvh_.depth >= kTailDepth && !work_counters_ ? kTailLanes : 0;
     st.spill = need > st.shared ? spill.p : nullptr;
     return st;
 }

@@ -37,12 +37,6 @@ namespace pt {
 
 namespace {
 
-__device__ __forceinline__ unsigned lanemask_lt() {
-    unsigned m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
-
 // Warp-aggregated append: every lane of the full warp calls this; lanes with `want` get a
 // slot index, computed from one atomic per warp.
 __device__ __forceinline__ int warp_append(int* counter, bool want) {
@@ -354,6 +348,35 @@ __global__ void __maxnreg__(traversal_regs(W)) k_extend(const __grid_constant__ 
     RayPre r = make_raypre(V{0.f, 0.f, 0.f}, V{0.f, 0.f, 1.f});
     Hit h{FLT_MAX, 0.f, 0.f, kMissPrim};
     int root = p.sc.root;
+    float tmax = FLT_MAX;
+    // The query ended: write its hit to the ray's own slot, or trace the direction again (true).
+    auto finish = [&]() -> bool {
+        if (of) atomicOr(&p.stats->error, 1);
+        // a triangle at t = tMin is inside the continuation's range, a sphere is not (triangle.cu:34
+        // accepts t >= tMin, sphere.cu:16,29 need t > tMin)
+        if (retrace && !second && h.prim != kMissPrim &&
+            (h.t < kBounceTMin || (h.prim < 0 && h.t == kBounceTMin))) {
+            // the BSDF-direct ray stopped closer than the continuation's tMin: keep its hit for
+            // the emission term and trace the direction again from kBounceTMin
+            q.hitd[slot] = make_float4(h.t, h.b1, h.b2, __int_as_float(h.prim));
+            second = true;
+            tmin = kBounceTMin;
+            h = Hit{FLT_MAX, 0.f, 0.f, kMissPrim};
+            cur = B ? root : p.sc.root;
+            sp = 0;
+            of = 0;
+            alive = true;
+            return true;
+        }
+        q.hit[slot] = make_float4(second ? -h.t : h.t, h.b1, h.b2, __int_as_float(h.prim));
+        if (p.shape.sort_materials) {
+            const int key = material_class(p.sc, h.prim);
+            q.key[slot] = key;
+            atomicAdd(&s_class[key], 1);
+        }
+        slot = -1;
+        return false;
+    };
     bool more = true;  // warp-uniform: the queue may hold rays not yet taken
     for (;;) {
         if (more) {
@@ -389,37 +412,14 @@ __global__ void __maxnreg__(traversal_regs(W)) k_extend(const __grid_constant__ 
             }
         }
         // with no query left after a fetch, the queue is exhausted (more is false)
-        if (!__any_sync(0xffffffffu, alive)) break;
-        traverse_round<W, false, CNT>(p.sc.nodes, p.sc.prims, quant, spec, r, tmin, FLT_MAX, st, h, cur, pend, sp, alive,
+        const unsigned busy = __ballot_sync(0xffffffffu, alive);
+        if (busy == 0 || (!more && __popc(busy) <= p.stack.tail)) break;
+        traverse_round<W, false, CNT>(p.sc.nodes, p.sc.prims, quant, spec, r, tmin, tmax, st, h, cur, pend, sp, alive,
                                       hit_any, of, &work, Q == 2);
-        // a triangle at t = tMin is inside the continuation's range, a sphere is not (triangle.cu:34
-        // accepts t >= tMin, sphere.cu:16,29 need t > tMin)
-        if (slot >= 0 && !alive && retrace && !second && h.prim != kMissPrim &&
-            (h.t < kBounceTMin || (h.prim < 0 && h.t == kBounceTMin))) {
-            // the BSDF-direct ray stopped closer than the continuation's tMin: keep its hit for
-            // the emission term and trace the direction again from kBounceTMin
-            if (of) atomicOr(&p.stats->error, 1);
-            q.hitd[slot] = make_float4(h.t, h.b1, h.b2, __int_as_float(h.prim));
-            second = true;
-            tmin = kBounceTMin;
-            h = Hit{FLT_MAX, 0.f, 0.f, kMissPrim};
-            cur = B ? root : p.sc.root;
-            sp = 0;
-            pend = kEmptyChild;
-            of = 0;
-            alive = true;
-        }
-        if (slot >= 0 && !alive) {  // the query ended: write its hit to the ray's own slot
-            if (of) atomicOr(&p.stats->error, 1);
-            q.hit[slot] = make_float4(second ? -h.t : h.t, h.b1, h.b2, __int_as_float(h.prim));
-            if (p.shape.sort_materials) {
-                const int key = material_class(p.sc, h.prim);
-                q.key[slot] = key;
-                atomicAdd(&s_class[key], 1);
-            }
-            slot = -1;
-        }
+        if (slot >= 0 && !alive) finish();
     }
+    traverse_tail<W, false, CNT>(p.sc.nodes, p.sc.prims, quant, r, tmin, tmax, st, h, cur, sp, alive, hit_any, of,
+                                 slot >= 0, &work, Q == 2, false, finish);
     __syncthreads();
     // one atomic per class and block for the whole persistent loop
     if (p.shape.sort_materials && threadIdx.x < kMaterialClasses && s_class[threadIdx.x] > 0)
@@ -1008,6 +1008,26 @@ __global__ void __maxnreg__(traversal_regs(W)) k_shadow(const __grid_constant__ 
     float tmax = 0.f;
     RayPre r = make_raypre(V{0.f, 0.f, 0.f}, V{0.f, 0.f, 1.f});
     Hit h{0.f, 0.f, 0.f, kMissPrim};  // unused by any-hit queries
+    float tmin = kShadowTMin;
+    auto finish = [&]() -> bool {  // the query ended: occluded, or nothing left to visit
+        const int i = slot;
+        slot = -1;
+        if (of) atomicOr(&p.stats->error, 1);
+        if (!occ) {
+            const float4 c = p.sq.c[i];
+            const int path = tag_path(tag);
+            float4 l = p.L[path];
+            l.x += c.x;
+            l.y += c.y;
+            l.z += c.z;
+            p.L[path] = l;
+            if (p.guide_mode) {
+                const long long ti = train_index<B>(p, tag_scene(tag), path, wave_first, gfirst);
+                guide_account(p, ti, depth, 0.f, (c.x + c.y + c.z) * (1.f / 3.f), 0.f);
+            }
+        }
+        return false;
+    };
     bool more = true;  // warp-uniform: the queue may hold rays not yet taken
     for (;;) {
         if (more) {
@@ -1034,28 +1054,14 @@ __global__ void __maxnreg__(traversal_regs(W)) k_shadow(const __grid_constant__ 
                 }
             }
         }
-        if (!__any_sync(0xffffffffu, alive)) break;
-        traverse_round<W, true, CNT>(p.sc.nodes, p.sc.prims, quant, spec, r, kShadowTMin, tmax, st, h, cur, pend, sp, alive,
+        const unsigned busy = __ballot_sync(0xffffffffu, alive);
+        if (busy == 0 || (!more && __popc(busy) <= p.shadow_stack.tail)) break;
+        traverse_round<W, true, CNT>(p.sc.nodes, p.sc.prims, quant, spec, r, tmin, tmax, st, h, cur, pend, sp, alive,
                                      occ, of, &work, Q == 2, near);
-        if (slot >= 0 && !alive) {  // the query ended: occluded, or the stack ran empty
-            const int i = slot;
-            slot = -1;
-            if (of) atomicOr(&p.stats->error, 1);
-            if (!occ) {
-                const float4 c = p.sq.c[i];
-                const int path = tag_path(tag);
-                float4 l = p.L[path];
-                l.x += c.x;
-                l.y += c.y;
-                l.z += c.z;
-                p.L[path] = l;
-                if (p.guide_mode) {
-                    const long long ti = train_index<B>(p, tag_scene(tag), path, wave_first, gfirst);
-                    guide_account(p, ti, depth, 0.f, (c.x + c.y + c.z) * (1.f / 3.f), 0.f);
-                }
-            }
-        }
+        if (slot >= 0 && !alive) finish();
     }
+    traverse_tail<W, true, CNT>(p.sc.nodes, p.sc.prims, quant, r, tmin, tmax, st, h, cur, sp, alive, occ, of, slot >= 0,
+                                &work, Q == 2, near, finish);
     if (CNT) flush_work(work, &p.stats->shadow_nodes, &p.stats->shadow_prims);
 }
 
@@ -1678,6 +1684,23 @@ __global__ void __launch_bounds__(kQueryBlock)
     float tmin = 0.f, tmax = 0.f;
     RayPre r = make_raypre(V{0.f, 0.f, 0.f}, V{0.f, 0.f, 1.f});
     Hit h{0.f, 0.f, 0.f, kMissPrim};
+    auto finish = [&]() -> bool {
+        if (of) *flags = 1;  // every writer stores the same value
+        if (ANY) {
+            out.occluded[i] = occ ? 1 : 0;
+        } else {
+            const bool hit = h.prim != kMissPrim, tri = hit && h.prim >= 0;
+            out.prim_type[i] = !hit ? -1 : tri ? kTriangle : kSphere;
+            out.prim_id[i] = !hit ? -1 : tri ? h.prim : ~h.prim;
+            out.mat_id[i] = !hit ? -1 : tri ? __float_as_int(sc.tri[kTriF4 * h.prim].w) : sc.sph_mat[~h.prim];
+            out.t[i] = hit ? h.t : 0.f;
+            if (out.bary) {
+                out.bary[2 * (size_t)i] = tri ? h.b1 : 0.f;
+                out.bary[2 * (size_t)i + 1] = tri ? h.b2 : 0.f;
+            }
+        }
+        return false;
+    };
     for (;;) {
         if (more) {
             const unsigned idle = __ballot_sync(0xffffffffu, !alive);
@@ -1707,26 +1730,15 @@ __global__ void __launch_bounds__(kQueryBlock)
                 }
             }
         }
-        if (!__any_sync(0xffffffffu, alive)) break;
+        const unsigned busy = __ballot_sync(0xffffffffu, alive);
+        if (busy == 0 || (!more && __popc(busy) <= shape.tail)) break;
         const bool was = alive;
         traverse_round<W, ANY, false>(sc.nodes, sc.prims, quant, false, r, tmin, tmax, st, h, cur, pend, sp, alive, occ,
                                       of, nullptr, wt);
-        if (!was || alive) continue;
-        if (of) *flags = 1;  // every writer stores the same value
-        if (ANY) {
-            out.occluded[i] = occ ? 1 : 0;
-        } else {
-            const bool hit = h.prim != kMissPrim, tri = hit && h.prim >= 0;
-            out.prim_type[i] = !hit ? -1 : tri ? kTriangle : kSphere;
-            out.prim_id[i] = !hit ? -1 : tri ? h.prim : ~h.prim;
-            out.mat_id[i] = !hit ? -1 : tri ? __float_as_int(sc.tri[kTriF4 * h.prim].w) : sc.sph_mat[~h.prim];
-            out.t[i] = hit ? h.t : 0.f;
-            if (out.bary) {
-                out.bary[2 * (size_t)i] = tri ? h.b1 : 0.f;
-                out.bary[2 * (size_t)i + 1] = tri ? h.b2 : 0.f;
-            }
-        }
+        if (was && !alive) finish();
     }
+    traverse_tail<W, ANY, false>(sc.nodes, sc.prims, quant, r, tmin, tmax, st, h, cur, sp, alive, occ, of, alive, nullptr,
+                                 wt, false, finish);
 }
 
 // One thread per triangle: vertices (the material id in p0's fourth word) and normals.

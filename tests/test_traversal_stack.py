@@ -82,3 +82,36 @@ def test_query_arrays_may_overlap():
         assert np.array_equal(got, ref[k]), k
     assert np.array_equal(t[:n], ref["t"])
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width", [2, 4])
+def test_ties_when_queries_are_shared(oracle_lib, width):
+    """few long queries (fewer than a warp's worth: its idle lanes share them) among coincident
+    primitives: the scan's tie rules decide, across the lanes' parts of a query too"""
+    n = 1500
+    v, nrm = _parallel_sheets(n)
+    v, nrm = np.concatenate([v, v[::-1]]), np.concatenate([nrm, nrm[::-1]])  # every sheet twice
+    zs = np.repeat(np.arange(0, 15, 0.05, dtype=np.float32), 2)  # and spheres, twice, tangent to sheets
+    sph = np.stack([np.zeros_like(zs), np.zeros_like(zs), zs + np.float32(0.5), np.full_like(zs, 0.5)], 1)
+    s = pathed.Session(32, 32)
+    s.set_bvh(width, 1)
+    s.load_arrays(tri_vertices=v, tri_normals=nrm, tri_materials=np.zeros(2 * n, np.int32), spheres=sph,
+                  sphere_materials=np.zeros(len(sph), np.int32), material_types=[0], material_albedo=[[0.5, 0.5, 0.5]],
+                  material_emit=[[0, 0, 0]], material_ior=[1.0], material_alpha=[0.1])
+    assert s.counts().bvh_depth >= 6
+    osc = oracle_lib.scene(s.export_scene())
+    rng = np.random.default_rng(width)
+    for m in (1, 3, 17, 300):
+        o = np.zeros((m, 3), np.float32)
+        o[:, 2] = -1
+        d = np.tile(np.float32([0, 0, 1]), (m, 1))
+        tmin = (1 + 0.01 * rng.integers(0, n - 20, m)).astype(np.float32) - np.float32(0.003)
+        tmax = np.full(m, FLT_MAX, np.float32)
+        r, g = oracle_lib.trace(osc, o, d, tmin, tmax), s.trace_rays(o, d, tmin, tmax)
+        for k in ("prim_type", "prim_id", "t"):
+            assert np.array_equal(g[k], r[k]), (m, k)
+        t1 = tmin + rng.choice([0.002, 0.5], m).astype(np.float32)  # short ones find nothing
+        occ = s.occluded(o, d, tmin, t1)
+        assert np.array_equal(occ, (oracle_lib.trace(osc, o, d, tmin, t1)["prim_type"] >= 0).astype(np.int32)), m
+    s.close()
