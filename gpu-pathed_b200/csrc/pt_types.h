@@ -164,12 +164,12 @@ struct StackShape {
 };
 // What a tree may need: at most width - 1 children left behind per level.
 PT_HD int stack_need(int width, int depth) { return (width - 1) * (depth + 1); }
-// When a warp's last queries are shared out: on trees of at least six levels, below 17 queries. Frame ms
+// When a warp's last queries are shared out: on trees of at least six levels and 1024 primitives, below 17 queries. Frame ms
 // before -> with 4 / 8 / 16 / 24 queries: guided slit room 3.91 -> 3.68 / 3.62 / 3.53 / 3.52, mesh at 1080p
 // 25.3 -> 24.9 / 24.7 / 24.6 / 24.5, slit room 67.8 -> 67.1 / 66.9 / 66.7 / 66.7, progressive slit room
 // 4.41 -> 4.28 / 4.23 / 4.17 / 4.17. Shallow trees have no long queries: sharing cost the Cornell box at
 // 400x400 and 1 spp 4%.
-constexpr int kTailDepth = 6, kTailLanes = 16;
+constexpr int kTailDepth = 6, kTailPrims = 1024, kTailLanes = 16;
 // Entries per lane in shared memory. 12 of 8 bytes take 106 KB at the 1024 threads per SM that 64
 // registers leave resident, so the L1 keeps about 96 KB for nodes and leaf entries; few lanes go
 // deeper. Frame ms with 6 / 8 / 11 / 12 / 16 entries: mesh 28.6 / 27.9 / 27.7 / 27.6 / 27.9, slit room 77.5 / 76.4 /

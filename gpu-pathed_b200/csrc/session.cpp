@@ -865,7 +865,8 @@ StackShape Session::stack_shape(const DevBuf& spill, int threads) const {
     st.cap = test_stack_cap_ > 0 ? std::min(test_stack_cap_, need) : need;
     st.spill_stride = threads;
     // frames that count work keep each query on its own lane: the counts are the queries' own visits
-    st.tail = bvh_.depth >= kTailDepth && !work_counters_ ? kTailLanes : 0;
+    const bool large = bvh_.depth >= kTailDepth && scene_.num_tri() + scene_.num_sph() >= kTailPrims;
+    st.tail = large && !work_counters_ ? kTailLanes : 0;
     st.spill = need > st.shared ? spill.p : nullptr;
     return st;
 }
