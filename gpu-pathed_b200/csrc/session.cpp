@@ -41,6 +41,7 @@ Session::Session(int w, int h) : w_(w), h_(h) {
 Session::~Session() {
     if (dev_ready_) {
         cudaSetDevice(device_);
+        QueryPool::get().detach();
         if (stream_) cudaStreamSynchronize(stream_);
         if (copy_stream_) {
             cudaStreamSynchronize(copy_stream_);
@@ -76,7 +77,6 @@ Session::~Session() {
             cudaStreamDestroy(query_stream_);
         }
         if (h_stats_) cudaFreeHost(h_stats_);
-        if (h_pick_) cudaFreeHost(h_pick_);
     }
 }
 
@@ -140,14 +140,16 @@ int Session::ensure_device() {
     if ((r = check_cuda(cudaEventCreateWithFlags(&cls_fork_, cudaEventDisableTiming), "cudaEventCreate"))) return r;
     side_ = SideStream{side_stream_, side_shaded_.data(), side_shadowed_.data(), cls_streams_.data(), cls_fork_,
                        cls_done_.data()};
-    if ((r = check_cuda(cudaMallocHost((void**)&h_stats_, sizeof(FrameStats)), "cudaMallocHost"))) return r;
+    if ((r = check_cuda(cudaMallocHost((void**)&h_stats_, sizeof(FrameStats) + 2 * sizeof(int)), "cudaMallocHost")))
+        return r;
     std::memset(h_stats_, 0, sizeof(FrameStats));
-    if ((r = check_cuda(cudaMallocHost((void**)&h_pick_, 2 * sizeof(int)), "cudaMallocHost"))) return r;
+    h_pick_ = reinterpret_cast<int*>(h_stats_ + 1);
     if ((r = check_cuda(d_counters_.alloc(sizeof(WaveCounters)), "counters"))) return r;
     if ((r = check_cuda(d_stats_.alloc(sizeof(FrameStats)), "stats"))) return r;
     if ((r = check_cuda(d_dyn_.alloc(sizeof(FrameDyn)), "frame constants"))) return r;
     if ((r = check_cuda(cudaMallocHost((void**)&h_dyn_, sizeof(FrameDyn)), "cudaMallocHost"))) return r;
     dev_ready_ = true;
+    QueryPool::get().attach();
     return PT_OK;
 }
 
@@ -857,28 +859,33 @@ int Session::upload_scene() {
     return upload_materials();
 }
 
-// Stacks of `threads` lanes for the tree on the device, their global part in `spill`.
-StackShape Session::stack_shape(const DevBuf& spill, int threads) const {
+// The traversal stacks of one user: the closest-hit stage and the queries on stream_, the shadow stage
+// beside it, or the allocation-free queries on query_stream_. Their global parts lie one behind the other.
+StackShape Session::stack_shape(StackArea area) const {
     StackShape st{};
-    const int need = stack_need(bvh_.width, bvh_.depth);
+    const int need = stack_need(bvh_.width, bvh_.depth), lanes = num_sms_ * kStackLanes;
     st.shared = std::min(need, kStackShared);
     st.cap = test_stack_cap_ > 0 ? std::min(test_stack_cap_, need) : need;
-    st.spill_stride = threads;
+    st.spill_stride = area == kStaticStacks ? kStaticTraceMaxRays : lanes;
     // frames that count work keep each query on its own lane: the counts are the queries' own visits
     const bool large = bvh_.depth >= kTailDepth && scene_.num_tri() + scene_.num_sph() >= kTailPrims;
     st.tail = large && !work_counters_ ? kTailLanes : 0;
-    st.spill = need > st.shared ? spill.p : nullptr;
+    if (need > st.shared) {
+        const size_t deep = need - st.shared;
+        const size_t at = area == kMainStacks     ? 0
+                          : area == kShadowStacks ? deep * lanes * sizeof(int2)
+                                                  : deep * lanes * (sizeof(int2) + sizeof(int));
+        st.spill = d_spill_.as<char>() + at;
+    }
     return st;
 }
 
 int Session::ensure_stacks() {
     const int need = stack_need(bvh_.width, bvh_.depth);
     if (need <= kStackShared) return PT_OK;
-    int r;
-    const size_t deep = (size_t)(need - kStackShared), lanes = (size_t)num_sms_ * kSmThreads;
-    if ((r = check_cuda(d_spill_.alloc(deep * lanes * sizeof(int2)), "traversal stacks"))) return r;
-    if ((r = check_cuda(d_shadow_spill_.alloc(deep * lanes * sizeof(int)), "traversal stacks"))) return r;
-    return check_cuda(d_query_spill_.alloc(deep * kStaticTraceMaxRays * sizeof(int2)), "traversal stacks");
+    const size_t lanes = (size_t)num_sms_ * kStackLanes;
+    const size_t per_entry = lanes * (sizeof(int2) + sizeof(int)) + kStaticTraceMaxRays * sizeof(int2);
+    return check_cuda(d_spill_.alloc((need - kStackShared) * per_entry), "traversal stacks");
 }
 
 SceneDevice Session::scene_view() const {
@@ -1042,8 +1049,8 @@ int Session::render_async(int spp) {
         p.batch_pixel_base = d_batch_pixel_base_.as<long long>();
         p.num_scenes = (int)batch_.size();
     }
-    p.stack = stack_shape(d_spill_, num_sms_ * kSmThreads);
-    p.shadow_stack = stack_shape(d_shadow_spill_, num_sms_ * kSmThreads);
+    p.stack = stack_shape(kMainStacks);
+    p.shadow_stack = stack_shape(kShadowStacks);
     p.mma_test_polls = test_mma_polls_;
     p.num_sms = num_sms_;
     p.count_work = work_counters_;
@@ -1625,7 +1632,7 @@ int Session::hit_test(int x, int y, int* mat) {
     if (mats_dirty_ && (r = upload_materials())) return r;
     std::string err;
     if (!make_camera(camspec_, w_, h_, cam_, err)) return fail(PT_ERR_ARG, err);
-    StackShape stack = stack_shape(d_spill_, 32);  // one query: all of its entries in shared memory
+    StackShape stack = stack_shape(kMainStacks);  // one query: all of its entries in shared memory
     stack.shared = stack.cap = stack_need(bvh_.width, bvh_.depth);
     // the kernel writes the material and the overflow flag to page-locked memory: one launch, no copies
     if ((r = check_cuda(enqueue_hit_test(scene_view(), cam_, stack, x, y, h_pick_, h_pick_ + 1, stream_), "hit test")))
@@ -1649,7 +1656,7 @@ int Session::trace_rays(const float* o, const float* d, const float* tmin, const
     if (in_flight_ && (r = wait(nullptr))) return r;
     if (scene_dirty_ && (r = upload_scene())) return r;
     if (mats_dirty_ && (r = upload_materials())) return r;
-    const StackShape sd = stack_shape(d_spill_, num_sms_ * kSmThreads);
+    const StackShape sd = stack_shape(kMainStacks);
     if (level_bytes(std::min(sd.cap, bvh_.depth + 1), 128) > (size_t)kMaxStackBytesDefault)
         return fail(PT_ERR_SCENE, "BVH too deep for the traversal stack in shared memory");
     if (device_ptrs) {
@@ -1680,7 +1687,7 @@ int Session::trace_rays_static(const float* o, const float* d, const float* tmin
         return fail(PT_ERR_STATE,
                     "scene not resident on the device; make one allocating device call (render, trace, hit "
                     "test) after loading or editing the scene");
-    StackShape sd = stack_shape(d_query_spill_, kStaticTraceMaxRays);
+    StackShape sd = stack_shape(kStaticStacks);
     sd.cap = stack_need(bvh_.width, bvh_.depth);
     if (level_bytes(bvh_.depth + 1, 128) > (size_t)kMaxStackBytesDefault)
         return fail(PT_ERR_SCENE, "BVH too deep for the traversal stack in shared memory");

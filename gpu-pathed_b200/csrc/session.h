@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -57,15 +58,33 @@ struct HostHits {  // closest hit: the five arrays (bary may be null); any hit: 
 };
 constexpr int kQueryWorkers = 8;
 struct QueryStaging {  // one chunk of page-locked and device memory and a stream per worker
+    int device;
     void* host = nullptr;
     size_t host_bytes = 0;
     DevBuf dev;
     std::vector<cudaStream_t> streams;
-    QueryStaging() = default;
+    explicit QueryStaging(int d) : device(d) {}
     QueryStaging(const QueryStaging&) = delete;
     QueryStaging& operator=(const QueryStaging&) = delete;
     ~QueryStaging();
     cudaError_t ensure(int workers, size_t bytes_each);
+};
+// The staging of all sessions of the process: page-locking costs 0.5 ms per MB, ten times what a call
+// saves, so a call borrows a staging and gives it back. At most kQueryStagings lie idle (concurrent calls
+// beyond that make their own and free it); the last session on a device frees them.
+constexpr int kQueryStagings = 2;
+class QueryPool {
+public:
+    static QueryPool& get();
+    std::unique_ptr<QueryStaging> take(int device);
+    void give(std::unique_ptr<QueryStaging> s);
+    void attach();  // a session that may call
+    void detach();
+
+private:
+    std::mutex m_;
+    std::vector<std::unique_ptr<QueryStaging>> idle_;
+    int sessions_ = 0;
 };
 
 inline bool env_cuts_fit(int w, int h) { return w <= kCdfCutMax && h <= kCdfCutMax; }
@@ -219,7 +238,7 @@ private:
     int frames_ = 0;
     FrameStats last_stats_{};
     FrameStats* h_stats_ = nullptr;  // pinned
-    int* h_pick_ = nullptr;          // pinned: a hit test's material and overflow flag
+    int* h_pick_ = nullptr;          // pinned (behind h_stats_): a hit test's material and overflow flag
     // profiling
     int stage_timing_ = 0;
     int work_counters_ = 0;
@@ -342,11 +361,12 @@ private:
     int test_mma_polls_ = 0;
     // traversal stacks (dev_trace.cuh, LaneStack): the closest-hit stage and the queries on
     // stream_, the shadow stage beside it, and the allocation-free queries on query_stream_
-    DevBuf d_spill_, d_shadow_spill_, d_query_spill_;
+    DevBuf d_spill_;
+    enum StackArea { kMainStacks, kShadowStacks, kStaticStacks };
     int ensure_stacks();
-    QueryStaging query_;
     int host_query(const HostRays& rays, const HostHits& out);
-    StackShape stack_shape(const DevBuf& spill, int threads) const;
+    int host_query(const HostRays& rays, const HostHits& out, QueryStaging& staging);
+    StackShape stack_shape(StackArea area) const;
 };
 
 }  // namespace pt

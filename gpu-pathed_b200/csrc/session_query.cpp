@@ -5,7 +5,7 @@
 // for a single ray. Calls beyond one chunk are worked off by several host threads, each with its own
 // stream and staging: a thread copies a chunk's rays into its staging, queues copy, kernel and
 // copy back, and copies the results out while the other threads' chunks are on the bus and on
-// the GPU. The staging is bounded (kQueryWorkers chunks) and belongs to the session.
+// the GPU. The staging is bounded (kQueryWorkers chunks) and borrowed from the process's pool.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -18,9 +18,10 @@
 namespace pt {
 
 namespace {
-// Rays per chunk and threads: a call of 1M rays, in ms, with 8 threads and chunks of 8192 / 16384 / 32768 rays
-// 3.3 / 2.6 / 2.1, with 4 threads and 32768 3.3; 4.4 by whole-array copies on one thread.
-constexpr int kChunkRays = 32768;
+// Rays per chunk, with 8 threads: 1M / 200k / 33k closest hits in ms at 8192 rays 2.6 / 0.64 / 0.21, at 16384 2.1 /
+// 0.56 / 0.24, at 32768 2.0 / 0.8 / 0.29 (whole-array copies on one thread: 4.2 / 1.03 / 0.34). The staging, 0.9 MB per
+// thread, takes about 4 ms to page-lock, once per process.
+constexpr int kChunkRays = 16384;
 // Up to here the kernel reads and writes the staging itself: 42 us for one ray, 105 us before.
 constexpr int kDirectRays = 2048;
 constexpr size_t kInBytes = 32;     // origin, direction, tmin, tmax
@@ -38,6 +39,41 @@ QueryStaging::~QueryStaging() {
     for (cudaStream_t s : streams)
         if (s) cudaStreamDestroy(s);
     if (host) cudaFreeHost(host);
+}
+
+QueryPool& QueryPool::get() {
+    static QueryPool* p = new QueryPool;  // never destroyed: no CUDA calls while the process ends
+    return *p;
+}
+
+std::unique_ptr<QueryStaging> QueryPool::take(int device) {
+    {
+        std::lock_guard<std::mutex> lock(m_);
+        for (size_t i = 0; i < idle_.size(); i++)
+            if (idle_[i]->device == device) {
+                std::unique_ptr<QueryStaging> s = std::move(idle_[i]);
+                idle_.erase(idle_.begin() + i);
+                return s;
+            }
+    }
+    return std::unique_ptr<QueryStaging>(new QueryStaging(device));
+}
+
+void QueryPool::give(std::unique_ptr<QueryStaging> s) {
+    std::lock_guard<std::mutex> lock(m_);
+    if (sessions_ > 0 && (int)idle_.size() < kQueryStagings && s->host_bytes <= kQueryWorkers * chunk_bytes(kChunkRays))
+        idle_.push_back(std::move(s));
+}
+
+void QueryPool::attach() {
+    std::lock_guard<std::mutex> lock(m_);
+    sessions_++;
+}
+
+void QueryPool::detach() {
+    std::vector<std::unique_ptr<QueryStaging>> gone;
+    std::lock_guard<std::mutex> lock(m_);
+    if (--sessions_ == 0) gone.swap(idle_);
 }
 
 cudaError_t QueryStaging::ensure(int workers, size_t bytes_each) {
@@ -58,6 +94,13 @@ cudaError_t QueryStaging::ensure(int workers, size_t bytes_each) {
 }
 
 int Session::host_query(const HostRays& rays, const HostHits& out) {
+    std::unique_ptr<QueryStaging> staging = QueryPool::get().take(device_);
+    const int r = host_query(rays, out, *staging);
+    QueryPool::get().give(std::move(staging));  // nothing of it is in use: every worker has waited for its stream
+    return r;
+}
+
+int Session::host_query(const HostRays& rays, const HostHits& out, QueryStaging& staging) {
     const size_t n = (size_t)rays.n;
     const bool any = out.occluded != nullptr;
     // a chunk's results are written while later chunks' rays are unread: only when no arrays overlap
@@ -76,19 +119,20 @@ int Session::host_query(const HostRays& rays, const HostHits& out) {
     const int workers = std::min({chunks, kQueryWorkers, threads});
     const size_t each = chunk_bytes(chunk);
     int r;
-    if ((r = check_cuda(query_.ensure(workers, each), "query staging"))) return r;
+    if ((r = check_cuda(staging.ensure(workers, each), "query staging"))) return r;
 
     const SceneDevice sc = scene_view();
     const size_t deep = (size_t)std::max(0, stack_need(bvh_.width, bvh_.depth) - kStackShared);
-    const int lanes = num_sms_ * kSmThreads / workers / 128 * 128;  // each worker's part of the stacks' global memory
+    const int lanes = num_sms_ * kStackLanes / workers / 128 * 128;  // each worker's part of the stacks' global memory
     std::atomic<int> next{0};
     std::atomic<int> err{(int)cudaSuccess}, overflowed{0};
     auto work = [&](int w) {
         cudaError_t e = cudaSetDevice(device_);
-        char* h = static_cast<char*>(query_.host) + w * each;
-        char* d = query_.dev.as<char>() + w * each;
-        const cudaStream_t st = query_.streams[w];
-        StackShape stack = stack_shape(d_spill_, lanes);
+        char* h = static_cast<char*>(staging.host) + w * each;
+        char* d = staging.dev.as<char>() + w * each;
+        const cudaStream_t st = staging.streams[w];
+        StackShape stack = stack_shape(kMainStacks);
+        stack.spill_stride = lanes;
         if (stack.spill) stack.spill = static_cast<char*>(stack.spill) + (size_t)w * deep * lanes * sizeof(int2);
         for (int c; e == cudaSuccess && err.load() == (int)cudaSuccess && (c = next.fetch_add(1)) < chunks;) {
             const size_t at = c * chunk, m = std::min(chunk, n - at);

@@ -1382,11 +1382,13 @@ ShadowKernel shadow_kernel(const SceneDevice& sc) {
     return W >= 4 && sc.node_q ? k_shadow<W, CNT, B, (W >= 4 ? 1 : 0)> : k_shadow<W, CNT, B, 0>;
 }
 
-// Blocks of a persistent grid: shape.blocks_per_sm per SM, at most what stays resident.
-cudaError_t resident_grid(const void* kernel, int block, size_t smem, const FrameParams& p, int& grid) {
+// Blocks of a persistent grid: shape.blocks_per_sm per SM, at most what stays resident and has stacks.
+cudaError_t resident_grid(const void* kernel, int block, size_t smem, const FrameParams& p, const StackShape& stack,
+                          int& grid) {
     int per_sm = 0;
     const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
     grid = p.num_sms * std::max(1, std::min(per_sm, p.shape.blocks_per_sm));
+    grid = std::max(1, std::min(grid, stack.spill_stride / block));
     return e;
 }
 
@@ -1432,8 +1434,8 @@ cudaError_t enqueue_waves(const FrameParams& p_in, const WaveRange* waves, int n
     const ExtendKernel extend = extend_kernel<W, CNT, B>(p.sc);
     const ShadowKernel shadow = shadow_kernel<W, CNT, B>(p.sc);
     int grid_e = 0, grid_s = 0;
-    cudaError_t ge = resident_grid((const void*)extend, p.shape.block_extend, smem_e, p, grid_e);
-    if (ge == cudaSuccess) ge = resident_grid((const void*)shadow, p.shape.block_shadow, smem_s, p, grid_s);
+    cudaError_t ge = resident_grid((const void*)extend, p.shape.block_extend, smem_e, p, p.stack, grid_e);
+    if (ge == cudaSuccess) ge = resident_grid((const void*)shadow, p.shape.block_shadow, smem_s, p, p.shadow_stack, grid_s);
     if (ge != cudaSuccess) return ge;
     Marker mark{marks, stream};
     Marker smark{marks, sstream};  // the side stream's shadow stages
@@ -1655,7 +1657,7 @@ cudaError_t set_smem_w(size_t bytes) {
     return cudaSuccess;
 }
 
-// Caller-provided queries, persistent: a warp's first 32 rays are its own by its index in the
+// Caller-provided queries, persistent: a warp's first `share` rays are its own by its index in the
 // grid, later ones come from a cursor, taken (as in the closest-hit stage) whenever half the
 // warp's lanes are idle. flags[0]: the overflow flag, flags[1]: the cursor.
 constexpr int kQueryBlock = 128;
@@ -1672,14 +1674,15 @@ struct QueryHits {  // closest hit: the five arrays (bary may be null); any hit:
 template <int W, bool ANY>
 __global__ void __launch_bounds__(kQueryBlock)
     k_query(const __grid_constant__ SceneDevice sc, const __grid_constant__ StackShape shape,
-            const __grid_constant__ QueryRays rays, const __grid_constant__ QueryHits out, int* flags) {
+            const __grid_constant__ QueryRays rays, const __grid_constant__ QueryHits out, int* flags, int share) {
     extern __shared__ int2 stk[];
     using Stack = LaneStack<ANY>;
     const Stack st{reinterpret_cast<typename Stack::Entry*>(stk) + threadIdx.x, (int)blockDim.x, shape};
     const bool quant = W >= 4 && sc.node_q != 0, wt = sc.watertight != 0;
     const int lane = threadIdx.x & 31;
-    const int rest = gridDim.x * blockDim.x;  // first ray the cursor serves
-    int i = blockIdx.x * blockDim.x + threadIdx.x, cur = kEmptyChild, pend = kEmptyChild, sp = 0, of = 0;
+    const int rest = (int)(gridDim.x * blockDim.x >> 5) * share;  // first ray the cursor serves
+    int i = lane < share ? (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * share + lane : rays.n;
+    int cur = kEmptyChild, pend = kEmptyChild, sp = 0, of = 0;
     bool alive = false, occ = false, first = true, more = true;
     float tmin = 0.f, tmax = 0.f;
     RayPre r = make_raypre(V{0.f, 0.f, 0.f}, V{0.f, 0.f, 1.f});
@@ -1876,19 +1879,23 @@ cudaError_t enqueue_query(const SceneDevice& sc, const StackShape& stack, const 
                                              : nullptr;
     if (!kernel) return cudaErrorInvalidValue;
     const size_t smem = stack_bytes(stack, kQueryBlock, ANY ? sizeof(int) : sizeof(int2));
-    // a block per kQueryBlock rays, at most what stays resident and what the stacks' global part has room for
+    // at most what stays resident and what the stacks' global part has room for
     int per_sm = 0, dev = 0, sms = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kQueryBlock, smem);
     if (e != cudaSuccess || (e = cudaGetDevice(&dev)) != cudaSuccess ||
         (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return e;
-    const int need = (int)(((long long)rays.n + kQueryBlock - 1) / kQueryBlock);
-    const int grid = std::max(1, std::min({need, per_sm * sms, stack.spill_stride / kQueryBlock}));
+    const int most = std::max(1, std::min(per_sm * sms, stack.spill_stride / kQueryBlock)), warps = kQueryBlock / 32;
+    // 32 rays per warp, or (where long queries are shared out) down to 8: half-empty warps on all of the SMs
+    // answer a short call sooner (10k closest hits against 0.33M triangles 133 -> 123 us, 33k 290 -> 230)
+    const int even = (int)(((long long)rays.n + most * warps - 1) / (most * warps));
+    int share = stack.tail ? std::min(32, std::max(8, even)) : 32;
+    const int grid = (int)std::min<long long>(most, ((long long)rays.n + share * warps - 1) / (share * warps));
     SceneDevice a0 = sc;
     StackShape a1 = stack;
     QueryRays a2 = rays;
     QueryHits a3 = out;
-    void* args[] = {&a0, &a1, &a2, &a3, &flags};
+    void* args[] = {&a0, &a1, &a2, &a3, &flags, &share};
     return cudaLaunchKernel(kernel, dim3(grid), dim3(kQueryBlock), args, smem, stream);
 }
 }  // namespace

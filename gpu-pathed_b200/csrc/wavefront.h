@@ -30,7 +30,8 @@ struct ShadowQueue {
 };
 
 constexpr int kMaxDepthLimit = 64;
-constexpr int kSmThreads = 2048;  // resident threads per SM, at most
+// Lanes per SM with a traversal stack: what the traversal grids keep resident at 64 registers.
+constexpr int kStackLanes = 1024;
 
 // Device counters of one depth of a wave (zeroed at wave start). Every warp of a stage's grid
 // adds to the stage's cursor and to the queue lengths, and one L2 slice serves about 1.5 such
