@@ -390,7 +390,8 @@ int pt_hit_test(pt_session* s, int x, int y, int* material_id);
 /* Closest hit of n caller rays against the loaded scene, host arrays (parity entry for
  * World::hit, src/world.cu:5-41). o, d: 3 floats per ray. Outputs per ray: prim_type (0
  * triangle, 1 sphere, -1 miss), prim_id, mat_id (-1 on a miss), t. bary (2 per ray) may be
- * NULL. */
+ * NULL. Calls of more than 16384 rays are copied in and out by up to eight threads that the
+ * call starts and joins (pt_occluded likewise). */
 int pt_trace_rays(pt_session* s, const float* o, const float* d, const float* tmin, const float* tmax,
                   int n, int* prim_type, int* prim_id, int* mat_id, float* t, float* bary);
 /* Same with device pointers (no copies; arrays must be device memory of this device). */
@@ -498,8 +499,8 @@ int pt_set_watertight(pt_session* s, int on);
 
 /* Test hook for the device-error paths (no counterpart in the reference, whose gpuAssert exits
  * the process, include/macro_helper.h:10-19). stack_entries > 0 caps the traversal stack of
- * every query of the frames, pt_trace_rays and pt_occluded at that many entries (below the BVH
- * depth a query that needs more gives up); mma_polls > 0 limits the first wait of each
+ * every query of the frames, pt_trace_rays and pt_occluded at that many entries (a query that
+ * needs more gives up); mma_polls > 0 limits the first wait of each
  * tensor-core inference layer (pt_set_guide_inference(1)) to that many non-blocking polls, so
  * it gives up while the layer's MMA runs (a bounded drain still waits for that MMA before the
  * kernel releases tensor memory). Either way the kernel sets its error flag and returns; the
