@@ -365,7 +365,8 @@ private:
     enum StackArea { kMainStacks, kShadowStacks, kStaticStacks };
     int ensure_stacks();
     int host_query(const HostRays& rays, const HostHits& out);
-    int host_query(const HostRays& rays, const HostHits& out, QueryStaging& staging);
+    int whole_query(const HostRays& rays, const HostHits& out);
+    int staged_query(const HostRays& rays, const HostHits& out, size_t chunk_rays, QueryStaging& staging);
     StackShape stack_shape(StackArea area) const;
 };
 

@@ -5,7 +5,8 @@
 // for a single ray. Calls beyond one chunk are worked off by several host threads, each with its own
 // stream and staging: a thread copies a chunk's rays into its staging, queues copy, kernel and
 // copy back, and copies the results out while the other threads' chunks are on the bus and on
-// the GPU. The staging is bounded (kQueryWorkers chunks) and borrowed from the process's pool.
+// the GPU. The staging is bounded (kQueryWorkers chunks) and borrowed from the process's pool. Large
+// calls whose arrays overlap are not cut up: whole_query copies each array once.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -21,7 +22,9 @@ namespace {
 // Rays per chunk, with 8 threads: 1M / 200k / 33k closest hits in ms at 8192 rays 2.6 / 0.64 / 0.21, at 16384 2.1 /
 // 0.56 / 0.24, at 32768 2.0 / 0.8 / 0.29 (whole-array copies on one thread: 4.2 / 1.03 / 0.34). The staging, 0.9 MB per
 // thread, takes about 4 ms to page-lock, once per process.
-constexpr int kChunkRays = 16384;
+constexpr size_t kChunkRays = 16384;
+// Largest call staged in one piece: its staging stays within the pool's (kQueryWorkers chunks).
+constexpr size_t kOnePiece = 4 * kChunkRays;
 // Up to here the kernel reads and writes the staging itself: 42 us for one ray, 105 us before.
 constexpr int kDirectRays = 2048;
 constexpr size_t kInBytes = 32;     // origin, direction, tmin, tmax
@@ -29,10 +32,31 @@ constexpr size_t kFlagBytes = 16;   // overflow flag, work cursor
 constexpr size_t kOutBytes = 24;    // type, primitive, material, t, barycentrics
 size_t chunk_bytes(size_t n) { return (n * (kInBytes + kOutBytes) + kFlagBytes + 255) & ~(size_t)255; }
 
-bool overlap(const void* a, size_t na, const void* b, size_t nb) {
-    const char *x = static_cast<const char*>(a), *y = static_cast<const char*>(b);
-    return a && b && x < y + nb && y < x + na;
-}
+struct Array {  // one of a call's arrays, null where the call has none
+    const void* p;
+    size_t bytes;
+};
+struct Arrays {
+    Array in[4], out[6];
+    Arrays(const HostRays& r, const HostHits& h)
+        : in{{r.o, 12 * (size_t)r.n}, {r.d, 12 * (size_t)r.n}, {r.tmin, 4 * (size_t)r.n}, {r.tmax, 4 * (size_t)r.n}},
+          out{{h.prim_type, 4 * (size_t)r.n}, {h.prim_id, 4 * (size_t)r.n}, {h.mat_id, 4 * (size_t)r.n},
+              {h.t, 4 * (size_t)r.n}, {h.bary, 8 * (size_t)r.n}, {h.occluded, 4 * (size_t)r.n}} {}
+    // no array that is written shares memory with another one
+    bool apart() const {
+        for (int k = 0; k < 6; k++) {
+            for (const Array& a : in)
+                if (overlap(a, out[k])) return false;
+            for (int i = 0; i < k; i++)
+                if (overlap(out[i], out[k])) return false;
+        }
+        return true;
+    }
+    static bool overlap(const Array& a, const Array& b) {
+        const char *x = static_cast<const char*>(a.p), *y = static_cast<const char*>(b.p);
+        return x && y && x < y + b.bytes && y < x + a.bytes;
+    }
+};
 }  // namespace
 
 QueryStaging::~QueryStaging() {
@@ -94,26 +118,61 @@ cudaError_t QueryStaging::ensure(int workers, size_t bytes_each) {
 }
 
 int Session::host_query(const HostRays& rays, const HostHits& out) {
+    // a chunk's results are written while later chunks' rays are unread: only when no arrays overlap
+    const bool apart = Arrays(rays, out).apart();
+    if (!apart && (size_t)rays.n > kOnePiece) return whole_query(rays, out);
     std::unique_ptr<QueryStaging> staging = QueryPool::get().take(device_);
-    const int r = host_query(rays, out, *staging);
+    const int r = staged_query(rays, out, apart ? kChunkRays : kOnePiece, *staging);
     QueryPool::get().give(std::move(staging));  // nothing of it is in use: every worker has waited for its stream
     return r;
 }
 
-int Session::host_query(const HostRays& rays, const HostHits& out, QueryStaging& staging) {
+// The whole call at once: every array is copied by itself from and to the caller's memory, in stream
+// order, so all rays are read before a result is written.
+int Session::whole_query(const HostRays& rays, const HostHits& out) {
+    const size_t n = (size_t)rays.n;
+    const Arrays arrays(rays, out);
+    int r;
+    if ((r = check_cuda(d_scratch_.alloc(n * (kInBytes + kOutBytes) + kFlagBytes), "scratch"))) return r;
+    char* g = d_scratch_.as<char>();
+    float* f = reinterpret_cast<float*>(g);
+    int* flags = reinterpret_cast<int*>(g + kInBytes * n);
+    int* o = reinterpret_cast<int*>(g + kInBytes * n + kFlagBytes);
+    int flag = 0;
+    auto enqueue = [&]() -> cudaError_t {
+        cudaError_t e;
+        char* at = g;
+        for (const Array& a : arrays.in) {
+            if ((e = cudaMemcpyAsync(at, a.p, a.bytes, cudaMemcpyHostToDevice, stream_))) return e;
+            at += a.bytes;
+        }
+        if ((e = cudaMemsetAsync(flags, 0, kFlagBytes, stream_))) return e;
+        const StackShape stack = stack_shape(kMainStacks);
+        e = out.occluded ? enqueue_occluded(scene_view(), stack, f, f + 3 * n, f + 6 * n, f + 7 * n, rays.n, o, flags, stream_)
+                         : enqueue_trace_rays(scene_view(), stack, f, f + 3 * n, f + 6 * n, f + 7 * n, rays.n, o, o + n,
+                                              o + 2 * n, reinterpret_cast<float*>(o + 3 * n),
+                                              out.bary ? reinterpret_cast<float*>(o + 4 * n) : nullptr, flags, stream_);
+        if (e != cudaSuccess) return e;
+        at = reinterpret_cast<char*>(o);
+        for (const Array& a : arrays.out) {
+            if (!a.p) continue;
+            if ((e = cudaMemcpyAsync(const_cast<void*>(a.p), at, a.bytes, cudaMemcpyDeviceToHost, stream_))) return e;
+            at += a.bytes;
+        }
+        return cudaMemcpyAsync(&flag, flags, sizeof(int), cudaMemcpyDeviceToHost, stream_);
+    };
+    const cudaError_t e = enqueue();
+    const cudaError_t s = cudaStreamSynchronize(stream_);  // also after an error: no copy may land after the return
+    if ((r = check_cuda(e != cudaSuccess ? e : s, "ray query"))) return r;
+    if (flag) return fail(PT_ERR_DEVICE, "traversal stack overflow reported by a kernel");
+    return PT_OK;
+}
+
+// The call in chunks of at most `chunk_rays`, through `staging`.
+int Session::staged_query(const HostRays& rays, const HostHits& out, size_t chunk_rays, QueryStaging& staging) {
     const size_t n = (size_t)rays.n;
     const bool any = out.occluded != nullptr;
-    // a chunk's results are written while later chunks' rays are unread: only when no arrays overlap
-    const void* ins[4] = {rays.o, rays.d, rays.tmin, rays.tmax};
-    const size_t in_words[4] = {3, 3, 1, 1};
-    const void* outs[6] = {out.prim_type, out.prim_id, out.mat_id, out.t, out.bary, out.occluded};
-    const size_t out_words[6] = {1, 1, 1, 1, 2, 1};
-    bool apart = true;
-    for (int i = 0; i < 4; i++)
-        for (int k = 0; k < 6; k++) apart = apart && !overlap(ins[i], 4 * n * in_words[i], outs[k], 4 * n * out_words[k]);
-    for (int i = 0; i < 6; i++)
-        for (int k = 0; k < i; k++) apart = apart && !overlap(outs[i], 4 * n * out_words[i], outs[k], 4 * n * out_words[k]);
-    const size_t chunk = apart ? std::min<size_t>(n, kChunkRays) : n;
+    const size_t chunk = std::min(n, chunk_rays);
     const int chunks = (int)((n + chunk - 1) / chunk);
     const int threads = std::max(1, (int)std::thread::hardware_concurrency() / 2);
     const int workers = std::min({chunks, kQueryWorkers, threads});
