@@ -6,7 +6,7 @@
 // stream and staging: a thread copies a chunk's rays into its staging, queues copy, kernel and
 // copy back, and copies the results out while the other threads' chunks are on the bus and on
 // the GPU. The staging is bounded (kQueryWorkers chunks) and borrowed from the process's pool. Large
-// calls whose arrays overlap are not cut up: whole_query copies each array once.
+// calls whose arrays overlap, or are page-locked already, are not cut up: whole_query copies each array once.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -51,6 +51,20 @@ struct Arrays {
                 if (overlap(out[i], out[k])) return false;
         }
         return true;
+    }
+    // every array is page-locked memory of the caller's
+    bool locked() const {
+        for (const Array& a : in)
+            if (!locked(a)) return false;
+        for (const Array& a : out)
+            if (a.p && !locked(a)) return false;
+        return true;
+    }
+    static bool locked(const Array& a) {
+        cudaPointerAttributes attr{};
+        if (cudaPointerGetAttributes(&attr, a.p) == cudaSuccess) return attr.type == cudaMemoryTypeHost;
+        cudaGetLastError();  // not an error of the call
+        return false;
     }
     static bool overlap(const Array& a, const Array& b) {
         const char *x = static_cast<const char*>(a.p), *y = static_cast<const char*>(b.p);
@@ -118,9 +132,13 @@ cudaError_t QueryStaging::ensure(int workers, size_t bytes_each) {
 }
 
 int Session::host_query(const HostRays& rays, const HostHits& out) {
+    const Arrays arrays(rays, out);
     // a chunk's results are written while later chunks' rays are unread: only when no arrays overlap
-    const bool apart = Arrays(rays, out).apart();
+    const bool apart = arrays.apart();
     if (!apart && (size_t)rays.n > kOnePiece) return whole_query(rays, out);
+    // the bus reads and writes page-locked arrays as they are: 33k / 200k / 1M closest hits in ms 0.18 / 0.43 / 1.5,
+    // staged 0.37 / 0.53 / 2.0; up to one chunk the staging's single copies win (10k: 0.10, one copy per array 0.12)
+    if ((size_t)rays.n > kChunkRays && arrays.locked()) return whole_query(rays, out);
     std::unique_ptr<QueryStaging> staging = QueryPool::get().take(device_);
     const int r = staged_query(rays, out, apart ? kChunkRays : kOnePiece, *staging);
     QueryPool::get().give(std::move(staging));  // nothing of it is in use: every worker has waited for its stream

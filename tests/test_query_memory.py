@@ -50,6 +50,50 @@ def test_results_over_rays(n):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 16384, 16385, 200003])
+@pytest.mark.parametrize("pageable", [None, 0, 8])  # which of the nine arrays is not page-locked
+def test_page_locked_arrays(n, pageable):
+    import torch
+
+    s = _session()
+    rays = seeded_rays(s.export_scene(), n + 2, seed=n)
+    rays = [a[:n].copy() for a in rays]
+    ref = _hits(n)
+    _trace(s, *rays, ref, n)
+    own = [torch.from_numpy(a) if i == pageable else torch.from_numpy(a).pin_memory()
+           for i, a in enumerate(rays + _hits(n))]
+    got = [a.numpy() for a in own]
+    _trace(s, *got[:4], got[4:], n)
+    for a, b in zip(got[4:], ref):
+        assert np.array_equal(a, b)
+    got[4][:] = 7
+    s._check(pathed.lib.pt_occluded(s._h, *[a.ctypes.data for a in got[:4]], n, got[4].ctypes.data))
+    assert np.array_equal(got[4], (ref[0] >= 0).astype(np.int32))
+    s.close()
+
+
+@pytest.mark.gpu
+def test_page_locked_arrays_are_copied_straight():
+    """A large call on page-locked arrays leaves the copies to the GPU: the profiler's copies are one per
+    array, not one per staged chunk."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    n = 200003
+    s = _session()
+    own = [torch.from_numpy(a.copy()).pin_memory() for a in [*seeded_rays(s.export_scene(), n, seed=3), *_hits(n)]]
+    arrays = [a.numpy() for a in own]
+    _trace(s, *arrays[:4], arrays[4:], n)
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        _trace(s, *arrays[:4], arrays[4:], n)
+        torch.cuda.synchronize()
+    copies = {e.key: e.count for e in p.key_averages() if "Memcpy" in e.key}
+    assert sum(c for k, c in copies.items() if "HtoD" in k) == 4, copies
+    assert sum(c for k, c in copies.items() if "DtoH" in k) == 6, copies  # and the overflow flag
+    s.close()
+
+
+@pytest.mark.gpu
 def test_overlapping_arrays_cost_no_page_locking():
     """A large call whose results go over its rays takes as long as its copies and kernel do (about twice
     the separate arrays' time on a B200), not the 26 times that page-locking a staging of its size took."""
