@@ -2,7 +2,7 @@
 //
 // Rays and results pass through page-locked staging, one copy in and one out per chunk. Copies
 // from and to the caller's pageable arrays, one per array, held these calls at 15 GB/s, 0.1 ms even
-// for a single ray. Calls beyond one chunk are worked off by several host threads, each with its own
+// for a single ray. Calls beyond four chunks are worked off by several host threads, each with its own
 // stream and staging: a thread copies a chunk's rays into its staging, queues copy, kernel and
 // copy back, and copies the results out while the other threads' chunks are on the bus and on
 // the GPU. The staging is bounded (kQueryWorkers chunks) and borrowed from the process's pool. Large
@@ -23,7 +23,10 @@ namespace {
 // 0.56 / 0.24, at 32768 2.0 / 0.8 / 0.29 (whole-array copies on one thread: 4.2 / 1.03 / 0.34). The staging, 0.9 MB per
 // thread, takes about 4 ms to page-lock, once per process.
 constexpr size_t kChunkRays = 16384;
-// Largest call staged in one piece: its staging stays within the pool's (kQueryWorkers chunks).
+// Up to here a call is one piece, staged by the calling thread: starting threads and their first CUDA call cost more
+// than they save. 17k / 33k / 50k / 66k / 100k closest hits in ms in one piece 0.15 / 0.23 / 0.30 / 0.37 / 0.51, in
+// chunks on several threads 0.17 / 0.37 / 0.46 / 0.36 / 0.36 (whole-array copies 0.22 / 0.27 / 0.36 / 0.41 / 0.55). The
+// staging of such a piece stays within the pool's (kQueryWorkers chunks).
 constexpr size_t kOnePiece = 4 * kChunkRays;
 // Up to here the kernel reads and writes the staging itself: 42 us for one ray, 105 us before.
 constexpr int kDirectRays = 2048;
@@ -140,7 +143,7 @@ int Session::host_query(const HostRays& rays, const HostHits& out) {
     // staged 0.37 / 0.53 / 2.0; up to one chunk the staging's single copies win (10k: 0.10, one copy per array 0.12)
     if ((size_t)rays.n > kChunkRays && arrays.locked()) return whole_query(rays, out);
     std::unique_ptr<QueryStaging> staging = QueryPool::get().take(device_);
-    const int r = staged_query(rays, out, apart ? kChunkRays : kOnePiece, *staging);
+    const int r = staged_query(rays, out, (size_t)rays.n <= kOnePiece ? kOnePiece : kChunkRays, *staging);
     QueryPool::get().give(std::move(staging));  // nothing of it is in use: every worker has waited for its stream
     return r;
 }
@@ -194,7 +197,8 @@ int Session::staged_query(const HostRays& rays, const HostHits& out, size_t chun
     const int chunks = (int)((n + chunk - 1) / chunk);
     const int threads = std::max(1, (int)std::thread::hardware_concurrency() / 2);
     const int workers = std::min({chunks, kQueryWorkers, threads});
-    const size_t each = chunk_bytes(chunk);
+    // whole chunks, so that longer and longer calls do not page-lock their staging anew each time
+    const size_t each = chunk_bytes(chunk <= kChunkRays ? chunk : (chunk + kChunkRays - 1) / kChunkRays * kChunkRays);
     int r;
     if ((r = check_cuda(staging.ensure(workers, each), "query staging"))) return r;
 

@@ -72,24 +72,35 @@ def test_page_locked_arrays(n, pageable):
     s.close()
 
 
-@pytest.mark.gpu
-def test_page_locked_arrays_are_copied_straight():
-    """A large call on page-locked arrays leaves the copies to the GPU: the profiler's copies are one per
-    array, not one per staged chunk."""
+def _copies(s, arrays, n):
+    """The copies to and from the GPU that one call makes."""
     import torch
     from torch.profiler import ProfilerActivity, profile
 
-    n = 200003
-    s = _session()
-    own = [torch.from_numpy(a.copy()).pin_memory() for a in [*seeded_rays(s.export_scene(), n, seed=3), *_hits(n)]]
-    arrays = [a.numpy() for a in own]
     _trace(s, *arrays[:4], arrays[4:], n)
     with profile(activities=[ProfilerActivity.CUDA]) as p:
         _trace(s, *arrays[:4], arrays[4:], n)
         torch.cuda.synchronize()
-    copies = {e.key: e.count for e in p.key_averages() if "Memcpy" in e.key}
-    assert sum(c for k, c in copies.items() if "HtoD" in k) == 4, copies
-    assert sum(c for k, c in copies.items() if "DtoH" in k) == 6, copies  # and the overflow flag
+    return tuple(sum(e.count for e in p.key_averages() if "Memcpy" in e.key and way in e.key) for way in ("HtoD", "DtoH"))
+
+
+@pytest.mark.gpu
+def test_page_locked_arrays_are_copied_straight():
+    """A large call on page-locked arrays leaves the copies to the GPU: one per array, not one per staged chunk."""
+    import torch
+
+    n = 200003
+    s = _session()
+    own = [torch.from_numpy(a.copy()).pin_memory() for a in [*seeded_rays(s.export_scene(), n, seed=3), *_hits(n)]]
+    assert _copies(s, [a.numpy() for a in own], n) == (4, 6)  # and the overflow flag
+    s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [2049, 16385, 33000, 65536])
+def test_medium_calls_are_staged_in_one_piece(n):
+    s = _session()
+    assert _copies(s, [*seeded_rays(s.export_scene(), n, seed=4), *_hits(n)], n) == (1, 1)
     s.close()
 
 
