@@ -55,19 +55,19 @@ struct Arrays {
         }
         return true;
     }
-    // every array is page-locked memory of the caller's
-    bool locked() const {
-        for (const Array& a : in)
-            if (!locked(a)) return false;
-        for (const Array& a : out)
-            if (a.p && !locked(a)) return false;
-        return true;
-    }
-    static bool locked(const Array& a) {
-        cudaPointerAttributes attr{};
-        if (cudaPointerGetAttributes(&attr, a.p) == cudaSuccess) return attr.type == cudaMemoryTypeHost;
-        cudaGetLastError();  // not an error of the call
-        return false;
+    // the arrays' memory: every one page-locked; one of them device memory, which the host cannot read
+    void memory(bool& locked, bool& device) const {
+        locked = true;
+        device = false;
+        auto look = [&](const Array& a) {
+            cudaPointerAttributes attr{};
+            if (!a.p) return;
+            if (cudaPointerGetAttributes(&attr, a.p) != cudaSuccess) cudaGetLastError();  // unknown: as any host memory
+            locked = locked && attr.type == cudaMemoryTypeHost;
+            device = device || attr.type == cudaMemoryTypeDevice;
+        };
+        for (const Array& a : in) look(a);
+        for (const Array& a : out) look(a);
     }
     static bool overlap(const Array& a, const Array& b) {
         const char *x = static_cast<const char*>(a.p), *y = static_cast<const char*>(b.p);
@@ -136,12 +136,15 @@ cudaError_t QueryStaging::ensure(int workers, size_t bytes_each) {
 
 int Session::host_query(const HostRays& rays, const HostHits& out) {
     const Arrays arrays(rays, out);
+    bool locked, device;
+    arrays.memory(locked, device);  // 0.1 us per array
+    if (device) return fail(PT_ERR_ARG, "device memory passed as a host array (pt_trace_rays_device takes it)");
     // a chunk's results are written while later chunks' rays are unread: only when no arrays overlap
     const bool apart = arrays.apart();
     if (!apart && (size_t)rays.n > kOnePiece) return whole_query(rays, out);
     // the bus reads and writes page-locked arrays as they are: 33k / 200k / 1M closest hits in ms 0.18 / 0.43 / 1.5,
     // staged 0.37 / 0.53 / 2.0; up to one chunk the staging's single copies win (10k: 0.10, one copy per array 0.12)
-    if ((size_t)rays.n > kChunkRays && arrays.locked()) return whole_query(rays, out);
+    if ((size_t)rays.n > kChunkRays && locked) return whole_query(rays, out);
     std::unique_ptr<QueryStaging> staging = QueryPool::get().take(device_);
     const int r = staged_query(rays, out, (size_t)rays.n <= kOnePiece ? kOnePiece : kChunkRays, *staging);
     QueryPool::get().give(std::move(staging));  // nothing of it is in use: every worker has waited for its stream

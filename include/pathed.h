@@ -390,8 +390,9 @@ int pt_hit_test(pt_session* s, int x, int y, int* material_id);
 /* Closest hit of n caller rays against the loaded scene, host arrays (parity entry for
  * World::hit, src/world.cu:5-41). o, d: 3 floats per ray. Outputs per ray: prim_type (0
  * triangle, 1 sphere, -1 miss), prim_id, mat_id (-1 on a miss), t. bary (2 per ray) may be
- * NULL. Calls of more than 16384 rays are copied in and out by up to eight threads that the
- * call starts and joins (pt_occluded likewise). */
+ * NULL. Device memory is refused (PT_ERR_ARG). Calls of more than 65536 rays are copied in and out
+ * by up to eight threads that the call starts and joins, unless all arrays are page-locked or some
+ * overlap (pt_occluded likewise). */
 int pt_trace_rays(pt_session* s, const float* o, const float* d, const float* tmin, const float* tmax,
                   int n, int* prim_type, int* prim_id, int* mat_id, float* t, float* bary);
 /* Same with device pointers (no copies; arrays must be device memory of this device). */

@@ -72,6 +72,28 @@ def test_page_locked_arrays(n, pageable):
     s.close()
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 3000, 70001])
+def test_device_memory_is_refused(n):
+    """an error, as before queries were staged, not a crash of the host's copy"""
+    import torch
+
+    s = _session()
+    arrays = [*seeded_rays(s.export_scene(), n + 2, seed=5), *_hits(n)]
+    arrays = [a[:2 * n].copy() for a in arrays]
+    for k in range(9):
+        ptr = [a.ctypes.data for a in arrays]
+        on_gpu = torch.from_numpy(arrays[k]).cuda()
+        ptr[k] = on_gpu.data_ptr()
+        with pytest.raises(pathed.PathedError):
+            s._check(pathed.lib.pt_trace_rays(s._h, *ptr[:4], n, *ptr[4:]))
+        if k < 5:
+            with pytest.raises(pathed.PathedError):
+                s._check(pathed.lib.pt_occluded(s._h, *ptr[:4], n, ptr[4]))
+    _trace(s, *arrays[:4], arrays[4:], n)  # the session goes on
+    s.close()
+
+
 def _copies(s, arrays, n):
     """The copies to and from the GPU that one call makes."""
     import torch
