@@ -1659,7 +1659,8 @@ cudaError_t set_smem_w(size_t bytes) {
 
 // Caller-provided queries, persistent: a warp's first `share` rays are its own by its index in the
 // grid, later ones come from a cursor, taken (as in the closest-hit stage) whenever half the
-// warp's lanes are idle. flags[0]: the overflow flag, flags[1]: the cursor.
+// warp's lanes are idle. TAIL: a warp's last queries are shared out among its lanes. flags[0]: the
+// overflow flag, flags[1]: the cursor.
 constexpr int kQueryBlock = 128;
 constexpr int kQueryRefill = 16;
 struct QueryRays {
@@ -1671,7 +1672,7 @@ struct QueryHits {  // closest hit: the five arrays (bary may be null); any hit:
     float *t, *bary;
     int* occluded;
 };
-template <int W, bool ANY>
+template <int W, bool ANY, bool TAIL>
 __global__ void __launch_bounds__(kQueryBlock)
     k_query(const __grid_constant__ SceneDevice sc, const __grid_constant__ StackShape shape,
             const __grid_constant__ QueryRays rays, const __grid_constant__ QueryHits out, int* flags, int share) {
@@ -1734,14 +1735,15 @@ __global__ void __launch_bounds__(kQueryBlock)
             }
         }
         const unsigned busy = __ballot_sync(0xffffffffu, alive);
-        if (busy == 0 || (!more && __popc(busy) <= shape.tail)) break;
+        if (busy == 0 || (TAIL && !more && __popc(busy) <= shape.tail)) break;
         const bool was = alive;
         traverse_round<W, ANY, false>(sc.nodes, sc.prims, quant, false, r, tmin, tmax, st, h, cur, pend, sp, alive, occ,
                                       of, nullptr, wt);
         if (was && !alive) finish();
     }
-    traverse_tail<W, ANY, false>(sc.nodes, sc.prims, quant, r, tmin, tmax, st, h, cur, sp, alive, occ, of, alive, nullptr,
-                                 wt, false, finish);
+    if constexpr (TAIL)
+        traverse_tail<W, ANY, false>(sc.nodes, sc.prims, quant, r, tmin, tmax, st, h, cur, sp, alive, occ, of, alive,
+                                     nullptr, wt, false, finish);
 }
 
 // One thread per triangle: vertices (the material id in p0's fourth word) and normals.
@@ -1869,27 +1871,51 @@ cudaError_t configure_traversal_smem(size_t bytes) {
 }
 
 namespace {
+template <bool ANY, bool TAIL>
+const void* query_kernel(int width) {
+    switch (width) {
+        case 2: return (const void*)k_query<2, ANY, TAIL>;
+        case 4: return (const void*)k_query<4, ANY, TAIL>;
+        case 8: return (const void*)k_query<8, ANY, TAIL>;
+        default: return nullptr;
+    }
+}
+
+// A warp starts with as many rays as spread the call over the resident warps, 8 at the least and 32 at the most:
+// half-empty warps on all of the SMs answer a short call sooner (closest hits, kernel us with 32 / 16 / 8 rays per
+// warp: 1000 against 82k triangles 54 / 50 / 46, against the Cornell box 12 / 11 / 11).
+constexpr int kQueryShare = 8;
+// Calls of fewer rays do not share their last queries, and run a kernel without that code: a warp's few rays end
+// nearly together, and the rounds that share cost more than they save. Mean us of a call in the slit room (1.31M
+// triangles) with one ray per lane and no sharing, as before sharing / shared / not, width 4: 300 rays 56 / 62 / 53,
+// 800 66 / 70 / 63, 2000 76 / 74 / 74, 4000 89 / 78 / 90; width 8: 300 53 / 62 / 52, 800 63 / 72 / 65, 2000 71 / 73 /
+// 75, 4000 83 / 81 / 88. Among 82k triangles in the open, where most rays miss, width 4: 300 67 / 57 / 60, 800 77 /
+// 59 / 69, 2000 82 / 60 / 73.
+constexpr int kQueryTailRays = 1024;
 template <bool ANY>
 cudaError_t enqueue_query(const SceneDevice& sc, const StackShape& stack, const QueryRays& rays, const QueryHits& out,
                           int* flags, cudaStream_t stream) {
     if (rays.n <= 0) return cudaSuccess;
-    const void* kernel = sc.bvh_width == 2   ? (const void*)k_query<2, ANY>
-                         : sc.bvh_width == 4 ? (const void*)k_query<4, ANY>
-                         : sc.bvh_width == 8 ? (const void*)k_query<8, ANY>
-                                             : nullptr;
+    const bool tail = stack.tail > 0 && rays.n >= kQueryTailRays;
+    const void* kernel = tail ? query_kernel<ANY, true>(sc.bvh_width) : query_kernel<ANY, false>(sc.bvh_width);
     if (!kernel) return cudaErrorInvalidValue;
     const size_t smem = stack_bytes(stack, kQueryBlock, ANY ? sizeof(int) : sizeof(int2));
-    // at most what stays resident and what the stacks' global part has room for
-    int per_sm = 0, dev = 0, sms = 0;
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kQueryBlock, smem);
-    if (e != cudaSuccess || (e = cudaGetDevice(&dev)) != cudaSuccess ||
-        (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+    constexpr int warps = kQueryBlock / 32;
+    int dev = 0, sms = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess || (e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
         return e;
-    const int most = std::max(1, std::min(per_sm * sms, stack.spill_stride / kQueryBlock)), warps = kQueryBlock / 32;
-    // 32 rays per warp, or (where long queries are shared out) down to 8: half-empty warps on all of the SMs
-    // answer a short call sooner (10k closest hits against 0.33M triangles 133 -> 123 us, 33k 290 -> 230)
+    // at most what stays resident (one block per SM always does) and what the stacks' global part has room for
+    int most = sms;
+    if (rays.n > (long long)sms * warps * kQueryShare) {
+        int per_sm = 0;
+        if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kQueryBlock, smem)) != cudaSuccess)
+            return e;
+        most = per_sm * sms;
+    }
+    most = std::max(1, std::min(most, stack.spill_stride / kQueryBlock));
     const int even = (int)(((long long)rays.n + most * warps - 1) / (most * warps));
-    int share = stack.tail ? std::min(32, std::max(8, even)) : 32;
+    int share = std::min(32, std::max(kQueryShare, even));
     const int grid = (int)std::min<long long>(most, ((long long)rays.n + share * warps - 1) / (share * warps));
     SceneDevice a0 = sc;
     StackShape a1 = stack;
