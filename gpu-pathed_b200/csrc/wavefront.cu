@@ -314,11 +314,15 @@ __global__ void __launch_bounds__(kRaySortBlock) k_ray_scatter(const __grid_cons
 // queries ended. With kSpeculateExtend set, traverse_round parks each lane's first leaf and
 // keeps descending while another lane of the warp still searches for one.
 // 64 registers keep 8 blocks of 128 threads resident; left to itself the compiler takes 76 (7 blocks;
-// mesh 28.4 ms against 27.6, slit room 79.1 against 75.7). Width 8 spills at 64.
-__host__ __device__ constexpr int traversal_regs(int width) { return width == 8 ? 80 : 64; }
+// mesh 28.4 ms against 27.6, slit room 79.1 against 75.7). Width 8 spills at 64: 80, and 72 on quantized
+// nodes, whose planes are decoded one at a time (the kernels before took 70 to 72 there, so that blocks of up
+// to 896 threads launch: 7 warps in each quarter of an SM, where 80 registers leave room for 6, 768 threads).
+__host__ __device__ constexpr int traversal_regs(int width, int q, bool count) {
+    return width < 8 ? 64 : q == 1 && !count ? 72 : 80;
+}
 
 template <int W, bool CNT, bool B, int Q>
-__global__ void __maxnreg__(traversal_regs(W)) k_extend(const __grid_constant__ FrameParams p, int depth,
+__global__ void __maxnreg__(traversal_regs(W, Q, CNT)) k_extend(const __grid_constant__ FrameParams p, int depth,
                                                                 long long wave_first) {
     extern __shared__ int2 stk[];
     const LaneStack<false> st{stk + threadIdx.x, (int)blockDim.x, p.stack};
@@ -990,7 +994,7 @@ __global__ void __maxnreg__(shade_class_regs(CLS)) k_shade_class(const __grid_co
 }
 
 template <int W, bool CNT, bool B, int Q>
-__global__ void __maxnreg__(traversal_regs(W)) k_shadow(const __grid_constant__ FrameParams p, int depth,
+__global__ void __maxnreg__(traversal_regs(W, Q, CNT)) k_shadow(const __grid_constant__ FrameParams p, int depth,
                                                                 long long wave_first, long long gfirst) {
     extern __shared__ int stk_any[];
     const LaneStack<true> st{stk_any + threadIdx.x, (int)blockDim.x, p.shadow_stack};
@@ -1387,9 +1391,11 @@ cudaError_t resident_grid(const void* kernel, int block, size_t smem, const Fram
                           int& grid) {
     int per_sm = 0;
     const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorLaunchOutOfResources;  // the block needs more registers than an SM has
     grid = p.num_sms * std::max(1, std::min(per_sm, p.shape.blocks_per_sm));
     grid = std::max(1, std::min(grid, stack.spill_stride / block));
-    return e;
+    return cudaSuccess;
 }
 
 using ShadeKernel = void (*)(FrameParams, int, long long, long long);
