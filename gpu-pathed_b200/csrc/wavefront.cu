@@ -1869,11 +1869,22 @@ cudaError_t configure_guide_infer() {
     return cudaFuncSetAttribute(k_guide_infer<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kInferSmemBytes);
 }
 
+// The limit is a property of the kernels on a device, which all sessions of the process share: it is only raised, so
+// that no session lowers it under another's frames.
 cudaError_t configure_traversal_smem(size_t bytes) {
-    cudaError_t e;
+    static std::mutex mutex;
+    static std::vector<size_t> limit;  // by device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mutex);
+    if (limit.size() <= (size_t)dev) limit.resize(dev + 1, 0);
+    if (bytes <= limit[dev]) return cudaSuccess;
     if ((e = set_smem_w<2>(bytes))) return e;
     if ((e = set_smem_w<4>(bytes))) return e;
-    return set_smem_w<8>(bytes);
+    if ((e = set_smem_w<8>(bytes))) return e;
+    limit[dev] = bytes;
+    return cudaSuccess;
 }
 
 namespace {

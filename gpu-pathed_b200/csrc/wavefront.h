@@ -261,7 +261,7 @@ cudaError_t build_prim_classes(const SceneDevice& sc, uint8_t* classes, cudaStre
 // Cut points (kCdfCuts + 1 per row) of `rows` CDFs of n <= kCdfCutMax values each.
 cudaError_t build_cdf_cuts(const float* cdf, int n, int rows, uint16_t* cuts, cudaStream_t stream);
 
-// Raise the dynamic shared-memory limit of the traversal kernels to `bytes`.
+// Raise the dynamic shared-memory limit of the traversal kernels on the current device to at least `bytes`.
 cudaError_t configure_traversal_smem(size_t bytes);
 // Opt the guide inference kernel into its dynamic shared memory (weights + 8 warps x 32 rows).
 cudaError_t configure_guide_infer();

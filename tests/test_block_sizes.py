@@ -33,3 +33,30 @@ def test_largest_blocks(width, option, largest):
     s.set_launch(block_extend=128, block_shadow=128)
     assert np.array_equal(_image(s), ref)
     s.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("graph", [1, 2])
+def test_sessions_of_different_blocks(graph):
+    """The kernels' shared-memory limit is the process's: a session of smaller blocks does not lower it under
+    another's frames."""
+    def session(block):
+        s = pathed.Session(61, 47)
+        s.load_config(0)
+        s.set_launch(block_extend=block, block_shadow=block, use_graph=graph)
+        return s
+
+    small = session(128)
+    ref = {spp: None for spp in (1, 2, 3)}
+    for spp in ref:
+        small.reset()
+        small.render(spp)
+        ref[spp] = small.readback().copy()
+    a, b = session(1024), session(512)
+    for spp in ref:  # another spp each time: the frame is launched, or captured, anew
+        for s in (a, b, a):
+            s.reset()
+            s.render(spp)
+            assert np.array_equal(s.readback(), ref[spp]), spp
+    for s in (small, a, b):
+        s.close()
