@@ -128,8 +128,9 @@ cudaError_t QueryStaging::ensure(int workers, size_t bytes_each) {
     }
     if ((e = dev.alloc(workers * bytes_each))) return e;
     while ((int)streams.size() < workers) {
-        streams.push_back(nullptr);
-        if ((e = cudaStreamCreateWithFlags(&streams.back(), cudaStreamNonBlocking))) return e;
+        cudaStream_t st = nullptr;
+        if ((e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking))) return e;
+        streams.push_back(st);
     }
     return cudaSuccess;
 }
@@ -147,7 +148,8 @@ int Session::host_query(const HostRays& rays, const HostHits& out) {
     if ((size_t)rays.n > kChunkRays && locked) return whole_query(rays, out);
     std::unique_ptr<QueryStaging> staging = QueryPool::get().take(device_);
     const int r = staged_query(rays, out, (size_t)rays.n <= kOnePiece ? kOnePiece : kChunkRays, *staging);
-    QueryPool::get().give(std::move(staging));  // nothing of it is in use: every worker has waited for its stream
+    // nothing of it is in use: every worker has waited for its stream; after an error it is freed
+    if (r == PT_OK) QueryPool::get().give(std::move(staging));
     return r;
 }
 
