@@ -41,7 +41,7 @@ Session::Session(int w, int h) : w_(w), h_(h) {
 Session::~Session() {
     if (dev_ready_) {
         cudaSetDevice(device_);
-        QueryPool::get().detach();
+        QueryPool::get().detach(device_);
         if (stream_) cudaStreamSynchronize(stream_);
         if (copy_stream_) {
             cudaStreamSynchronize(copy_stream_);
@@ -149,7 +149,7 @@ int Session::ensure_device() {
     if ((r = check_cuda(d_dyn_.alloc(sizeof(FrameDyn)), "frame constants"))) return r;
     if ((r = check_cuda(cudaMallocHost((void**)&h_dyn_, sizeof(FrameDyn)), "cudaMallocHost"))) return r;
     dev_ready_ = true;
-    QueryPool::get().attach();
+    QueryPool::get().attach(device_);
     return PT_OK;
 }
 

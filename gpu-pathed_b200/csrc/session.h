@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <map>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -70,21 +71,21 @@ struct QueryStaging {  // one chunk of page-locked and device memory and a strea
     cudaError_t ensure(int workers, size_t bytes_each);
 };
 // The staging of all sessions of the process: page-locking costs 0.5 ms per MB, ten times what a call
-// saves, so a call borrows a staging and gives it back. At most kQueryStagings lie idle (concurrent calls
-// beyond that make their own and free it); the last session on a device frees them.
+// saves, so a call borrows a staging and gives it back. At most kQueryStagings per device lie idle (concurrent
+// calls beyond that make their own and free it); the last session on a device frees them.
 constexpr int kQueryStagings = 2;
 class QueryPool {
 public:
     static QueryPool& get();
     std::unique_ptr<QueryStaging> take(int device);
     void give(std::unique_ptr<QueryStaging> s);
-    void attach();  // a session that may call
-    void detach();
+    void attach(int device);  // a session that may call
+    void detach(int device);
 
 private:
     std::mutex m_;
     std::vector<std::unique_ptr<QueryStaging>> idle_;
-    int sessions_ = 0;
+    std::map<int, int> sessions_;  // by device
 };
 
 inline bool env_cuts_fit(int w, int h) { return w <= kCdfCutMax && h <= kCdfCutMax; }

@@ -102,19 +102,26 @@ std::unique_ptr<QueryStaging> QueryPool::take(int device) {
 
 void QueryPool::give(std::unique_ptr<QueryStaging> s) {
     std::lock_guard<std::mutex> lock(m_);
-    if (sessions_ > 0 && (int)idle_.size() < kQueryStagings && s->host_bytes <= kQueryWorkers * chunk_bytes(kChunkRays))
+    int idle = 0;
+    for (const auto& i : idle_) idle += i->device == s->device;
+    if (sessions_[s->device] > 0 && idle < kQueryStagings && s->host_bytes <= kQueryWorkers * chunk_bytes(kChunkRays))
         idle_.push_back(std::move(s));
 }
 
-void QueryPool::attach() {
+void QueryPool::attach(int device) {
     std::lock_guard<std::mutex> lock(m_);
-    sessions_++;
+    sessions_[device]++;
 }
 
-void QueryPool::detach() {
-    std::vector<std::unique_ptr<QueryStaging>> gone;
+void QueryPool::detach(int device) {
+    std::vector<std::unique_ptr<QueryStaging>> gone;  // freed after the lock
     std::lock_guard<std::mutex> lock(m_);
-    if (--sessions_ == 0) gone.swap(idle_);
+    if (--sessions_[device] > 0) return;
+    for (size_t i = idle_.size(); i-- > 0;)
+        if (idle_[i]->device == device) {
+            gone.push_back(std::move(idle_[i]));
+            idle_.erase(idle_.begin() + i);
+        }
 }
 
 cudaError_t QueryStaging::ensure(int workers, size_t bytes_each) {

@@ -39,6 +39,8 @@ cudaError_t cudaGetLastError() { return cudaSuccess; }
 using namespace pt;
 
 int main() {
+    QueryPool& pool = QueryPool::get();
+    const size_t each = chunk_bytes(kChunkRays);
     {  // a stream that cannot be made leaves no null stream behind
         QueryStaging s(0);
         g_fail_stream = 2;
@@ -48,6 +50,45 @@ int main() {
         CHECK(s.streams.size() == 4);
         for (cudaStream_t st : s.streams) CHECK(st != nullptr);
     }
+    CHECK(g_host == 0 && g_dev == 0 && g_streams == 0);
+    auto filled = [&](int device, size_t bytes) {
+        std::unique_ptr<QueryStaging> s = pool.take(device);
+        s->ensure(1, bytes);
+        return s;
+    };
+    // no session: nothing is kept
+    pool.give(filled(0, 256));
+    CHECK(g_host == 0);
+    // each device keeps its own, as many as the pool allows
+    pool.attach(0);
+    pool.attach(0);
+    pool.attach(1);
+    std::vector<std::unique_ptr<QueryStaging>> out;
+    for (int k = 0; k < kQueryStagings + 1; k++) out.push_back(filled(0, each));
+    out.push_back(filled(1, each));
+    for (auto& s : out) pool.give(std::move(s));
+    CHECK(g_host == kQueryStagings + 1);
+    QueryStaging* one = nullptr;
+    {
+        std::unique_ptr<QueryStaging> s = pool.take(1);
+        CHECK(s->device == 1 && s->host_bytes == each);
+        one = s.get();
+        pool.give(std::move(s));
+        CHECK(pool.take(1).get() == one);  // freed here
+    }
+    CHECK(g_host == kQueryStagings);
+    // a staging larger than the pool's bound is not kept
+    pool.give(filled(1, kQueryWorkers * each + 256));
+    CHECK(g_host == kQueryStagings);
+    pool.give(filled(1, kQueryWorkers * each));
+    CHECK(g_host == kQueryStagings + 1);
+    // the last session of a device frees that device's, and no other's
+    pool.detach(0);
+    CHECK(g_host == kQueryStagings + 1);
+    pool.detach(0);
+    CHECK(g_host == 1);
+    CHECK(pool.take(1)->host_bytes == kQueryWorkers * each);
+    pool.detach(1);
     CHECK(g_host == 0 && g_dev == 0 && g_streams == 0);
     std::printf("ok\n");
     return 0;
