@@ -779,22 +779,29 @@ int Session::upload_scene() {
         if ((r = check_cuda(upload(d_prims_, bvh_.prims, stream_), "upload BVH primitives"))) return r;
     }
     if ((r = check_cuda(d_tri_.alloc((size_t)nt * kTriF4 * sizeof(float4)), "triangles"))) return r;
-    if (nt > 0) {  // the scene's own arrays, packed into records on the device
-        const size_t floats = (size_t)nt * 9;
-        if ((r = check_cuda(d_scratch_.alloc((2 * floats + nt) * 4), "scratch"))) return r;
+    // the scene's own arrays, packed into records on the device, a part at a time: the scratch memory stays with
+    // the session (20 MB; a mesh of 1.31M triangles would leave 100 MB in one piece)
+    constexpr int kPackTriangles = 1 << 18;
+    const size_t most = (size_t)std::min(nt, kPackTriangles);
+    if (nt > 0 && (r = check_cuda(d_scratch_.alloc(most * 19 * 4), "scratch"))) return r;
+    for (int first = 0; first < nt; first += kPackTriangles) {
+        const int m = std::min(nt - first, kPackTriangles);
+        const size_t at = 9 * (size_t)first, bytes = 9 * (size_t)m * 4;
         float* p = d_scratch_.as<float>();
-        if ((r = check_cuda(cudaMemcpyAsync(p, scene_.tri_p.data(), floats * 4, cudaMemcpyHostToDevice, stream_),
+        float* n = p + 9 * most;
+        int* mat = reinterpret_cast<int*>(n + 9 * most);
+        if ((r = check_cuda(cudaMemcpyAsync(p, scene_.tri_p.data() + at, bytes, cudaMemcpyHostToDevice, stream_),
                             "upload triangles")))
             return r;
-        if ((r = check_cuda(cudaMemcpyAsync(p + floats, scene_.tri_n.data(), floats * 4, cudaMemcpyHostToDevice,
-                                            stream_),
+        if ((r = check_cuda(cudaMemcpyAsync(n, scene_.tri_n.data() + at, bytes, cudaMemcpyHostToDevice, stream_),
                             "upload normals")))
             return r;
-        int* mat = reinterpret_cast<int*>(p + 2 * floats);
-        if ((r = check_cuda(cudaMemcpyAsync(mat, scene_.tri_mat.data(), (size_t)nt * 4, cudaMemcpyHostToDevice, stream_),
+        if ((r = check_cuda(cudaMemcpyAsync(mat, scene_.tri_mat.data() + first, (size_t)m * 4, cudaMemcpyHostToDevice,
+                                            stream_),
                             "upload triangle materials")))
             return r;
-        if ((r = check_cuda(pack_triangles(p, p + floats, mat, nt, d_tri_.as<float4>(), stream_), "pack triangles")))
+        if ((r = check_cuda(pack_triangles(p, n, mat, m, d_tri_.as<float4>() + kTriF4 * (size_t)first, stream_),
+                            "pack triangles")))
             return r;
     }
     if ((r = check_cuda(upload(d_sph_, scene_.sph, stream_), "upload spheres"))) return r;
