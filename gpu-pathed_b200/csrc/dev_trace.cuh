@@ -573,10 +573,11 @@ __device__ __forceinline__ void leaf_step(const float4* __restrict__ prims, cons
 // one; phase 2 tests the leaves. Waiting for the last searching lane left most of a warp idle on
 // incoherent rays (8 of 32 lanes active on the 1.31M-triangle mesh). Frame ms with phase 1
 // ending at the last lane / at waiting >= 1x / 2x / 4x / 8x searching: mesh 33.7 / 30.1 / 30.2 / 30.7 / 31.7, slit
-// room 86.7 / 82.6 / 81.8 / 81.5 / 82.3, spheres 25.7 / 26.0 / 25.9 / 25.8 / 25.8, Cornell 3.26 / 3.31 / 3.26 / 3.26 / 3.28. With `spec` (speculative traversal, Aila and Laine 2009), a lane
-// that reaches its first leaf parks it in `pend` and keeps descending while some lane of the
-// warp has found no leaf yet, so the node phase runs with fuller warps; the parked leaf is
-// tested in phase 2. Closest hits are the minimum of a total order, so the visiting order
+// room 86.7 / 82.6 / 81.8 / 81.5 / 82.3, spheres 25.7 / 26.0 / 25.9 / 25.8 / 25.8, Cornell 3.26 / 3.31 / 3.26 / 3.26 /
+// 3.28.
+// With `spec` (speculative traversal, Aila and Laine 2009), a lane that reaches its first leaf
+// parks it in `pend` and keeps descending while some lane of the warp has found no leaf yet, so
+// the node phase runs with fuller warps; the parked leaf is tested in phase 2. Closest hits are the minimum of a total order, so the visiting order
 // never changes a result; speculation only visits nodes that a tighter bound might have culled.
 template <int W, bool ANY, bool CNT>
 __device__ __forceinline__ void traverse_round(const float4* __restrict__ nodes, const float4* __restrict__ prims,
@@ -744,16 +745,12 @@ __device__ __forceinline__ void traverse_tail(const float4* __restrict__ nodes, 
 // lanes that carry a query). Lanes advance through internal nodes in one phase and test
 // leaves in the next, re-converging at each phase boundary (the while-while organisation of
 // Aila and Laine, HPG 2009), so leaf tests and node visits execute as coherent SIMT
-// instructions instead of drifting apart. Returns whether the query hit. Q: node format, 0 float
-// nodes, 1 quantized nodes (W >= 4), -1 read from the scene at run time.
-template <int W, bool ANY, bool CNT = false, int Q = -1>
-__device__ __forceinline__ bool traverse(const SceneDevice& sc, const RayPre& r, float tmin, float tmax, bool active,
-                                         const LaneStack<ANY>& st, Hit& best, int& overflow,
-                                         TraceWork* work = nullptr) {
-    const float4* __restrict__ nodes = sc.nodes;
-    const float4* __restrict__ prims = sc.prims;
-    const bool quant = Q < 0 ? (W >= 4 && sc.node_q != 0) : (W >= 4 && Q == 1);  // warp-uniform
-    const bool wt = sc.watertight != 0;
+// instructions instead of drifting apart. Closest hit, no refill: the queries that start and end
+// together (normals frames, the pick).
+template <int W>
+__device__ __forceinline__ void traverse(const SceneDevice& sc, const RayPre& r, float tmin, float tmax, bool active,
+                                         const LaneStack<false>& st, Hit& best, int& overflow) {
+    const bool quant = W >= 4 && sc.node_q != 0, wt = sc.watertight != 0;  // warp-uniform
     best.prim = kMissPrim;
     best.t = tmax;
     int sp = 0;
@@ -762,13 +759,8 @@ __device__ __forceinline__ bool traverse(const SceneDevice& sc, const RayPre& r,
     bool hit_any = false;
     int pend = kEmptyChild;
     while (__any_sync(0xffffffffu, alive))
-        traverse_round<W, ANY, CNT>(nodes, prims, quant, false, r, tmin, tmax, st, best, cur, pend, sp, alive, hit_any,
-                                    overflow, work, wt);
-    if (ANY) {
-        if (hit_any) best.prim = 0;
-        return hit_any;
-    }
-    return best.prim != kMissPrim;
+        traverse_round<W, false, false>(sc.nodes, sc.prims, quant, false, r, tmin, tmax, st, best, cur, pend, sp, alive,
+                                        hit_any, overflow, nullptr, wt);
 }
 
 }  // namespace pt

@@ -2,7 +2,7 @@
 // (src/renderers/path_tracer.cu:142-264) split into stages over SoA ray queues.
 //
 //   camera   one thread per path of the wave: PCG stream, generateRay, queue slot
-//   extend   persistent: closest hit for every queued ray (BVH, shared-memory stack)
+//   extend   persistent: closest hit for every queued ray (BVH; stacks in shared, then global memory)
 //   sort     optional: bucket the queue by material class (miss, Lambert, mirror, glass,
 //            Beckmann) so each warp of the shade stage runs one BSDF
 //   shade    persistent: emission with MIS, BSDF sample, emitter sample (NEE) -> shadow
@@ -129,7 +129,7 @@ __device__ __forceinline__ SceneLights scene_lights(const FrameParams& p, int si
 // draws, camera.h:40-61), its queue tag and the path's random state after the draws. k_camera
 // queues it; in frames that do not queue camera rays (p.cam_fused) the closest-hit and shade
 // stages of depth 0 each compute it from the path index instead: the same operations on the
-// same inputs, so both stages see the same ray, and no camera stage writes 56 bytes per path.
+// same inputs, so both stages see the same ray, and no camera stage writes 64 bytes of records per path.
 template <bool B>
 __device__ __forceinline__ void camera_path(const FrameParams& p, long long wave_first, int i, V& o, V& d,
                                             int& tag, uint64_t& st) {
@@ -1572,7 +1572,7 @@ __global__ void k_normals(const __grid_constant__ FrameParams p, int first_pixel
         const RayPre r = make_raypre(o, d);
         Hit h;
         int of = 0;
-        traverse<W, false>(p.sc, r, kCameraTMin, FLT_MAX, valid, st, h, of);
+        traverse<W>(p.sc, r, kCameraTMin, FLT_MAX, valid, st, h, of);
         if (!valid) continue;
         if (of) atomicOr(&p.stats->error, 1);
         float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1796,7 +1796,7 @@ __global__ void k_hit_test(SceneDevice sc, CameraParams cam, StackShape shape, i
     Hit h;
     int of = 0;
     // the whole warp enters the traversal; lane 0 carries the query and owns the stack
-    traverse<W, false>(sc, r, 0.f, FLT_MAX, threadIdx.x == 0, LaneStack<false>{stk, 1, shape}, h, of);
+    traverse<W>(sc, r, 0.f, FLT_MAX, threadIdx.x == 0, LaneStack<false>{stk, 1, shape}, h, of);
     if (threadIdx.x != 0) return;
     *overflow = of ? 1 : 0;
     if (h.prim == kMissPrim) *out = -1;
