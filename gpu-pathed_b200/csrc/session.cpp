@@ -862,6 +862,7 @@ int Session::upload_scene() {
     }
     if (batch_mode() && (r = upload_batch())) return r;
     if ((r = ensure_stacks())) return r;
+    if ((r = check_cuda(load_query_kernels(bvh_.width), "query kernels"))) return r;
     scene_dirty_ = false;
     return upload_materials();
 }

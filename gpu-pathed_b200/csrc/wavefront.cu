@@ -1943,6 +1943,13 @@ cudaError_t enqueue_query(const SceneDevice& sc, const StackShape& stack, const 
 }
 }  // namespace
 
+cudaError_t load_query_kernels(int width) {
+    cudaFuncAttributes attr;
+    for (const void* kernel : {query_kernel<false, false>(width), query_kernel<false, true>(width)})
+        if (const cudaError_t e = kernel ? cudaFuncGetAttributes(&attr, kernel) : cudaSuccess) return e;
+    return cudaSuccess;
+}
+
 cudaError_t enqueue_trace_rays(const SceneDevice& sc, const StackShape& stack, const float* o, const float* d,
                                const float* tmin, const float* tmax, int n, int* prim_type, int* prim_id,
                                int* mat_id, float* t, float* bary, int* flags, cudaStream_t stream) {

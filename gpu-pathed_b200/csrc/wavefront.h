@@ -281,6 +281,10 @@ cudaError_t enqueue_occluded(const SceneDevice& sc, const StackShape& stack, con
 cudaError_t enqueue_hit_test(const SceneDevice& sc, const CameraParams& cam, const StackShape& stack, int x, int y,
                              int* out_material, int* overflow, cudaStream_t stream);
 
+// Loads the closest-hit query kernels of a BVH width, which the runtime otherwise does at their first launch, waiting
+// for all work on the device: a query beside a frame in flight would wait for the frame.
+cudaError_t load_query_kernels(int width);
+
 // Closest-hit queries that allocate nothing: host rays in, host results out, staged through
 // a file-scope __device__ array of kStaticTraceMaxRays entries (see wavefront.cu). The
 // first call on a device looks the array's address up (cudaGetSymbolAddress) with that
